@@ -173,6 +173,32 @@ __device__ __forceinline__ bool push_absent(const AntSmem& s, Checklist& q, std:
     return absent;
 }
 
+// Appends the nodes of lanes 0, 1, ... (each lane its own `v`, taken when
+// `want`) that are not pending, in lane order: what one append_if_absent
+// after the other does (cuda/faco_device.cuh:81-92).  The wanted nodes are
+// distinct.  Returns the number appended.
+__device__ __forceinline__ std::uint32_t push_lanes(const AntSmem& s, Checklist& q, std::uint32_t n, std::uint32_t v,
+                                                    bool want, std::uint32_t lane, std::uint32_t* log,
+                                                    std::uint32_t log_cap) {
+    const bool absent = want && !test_bit(s.queued, v);
+    const unsigned m = __ballot_sync(kFull, absent);   // every lane has read its flag before one is set
+    if (absent) {
+        const std::uint32_t rank = __popc(m & ((1u << lane) - 1u));
+        std::uint32_t at = q.tail + rank;
+        if (at >= n) at -= n;
+        atomicOr(&s.queued[v >> 5], 1u << (v & 31u));
+        s.ring[at] = (node_t)v;
+        if (log && q.pushed + rank < log_cap) log[q.pushed + rank] = v;
+    }
+    const std::uint32_t count = __popc(m);
+    q.tail += count;
+    if (q.tail >= n) q.tail -= n;
+    q.pending += count;
+    q.pushed += count;
+    __syncwarp();
+    return count;
+}
+
 __device__ __forceinline__ std::uint32_t pop(const AntSmem& s, Checklist& q, std::uint32_t n,
                                              std::uint32_t lane) {
     const std::uint32_t a = s.ring[q.head];
@@ -637,83 +663,165 @@ __device__ __forceinline__ LsRow pop_with_row(const AntSmem& s, Checklist& q, st
 
 // Checklist 2-opt, best gain per popped node, reference tie/cap rules
 // (cpp/src/faco_cpu.cpp:148-217; cuda/faco_device.cuh:295-478).
-// kCompact (the batched-step variants, bound by instruction fetch): the four
-// pushes of a move through one copy of push_absent.
-template <bool kCompact = false>
+//
+// Up to kPopNodes nodes from the head of the checklist are evaluated
+// together.  About two pops in three find no move and then leave the tour as
+// it is, so the nodes up to and including the first one with a move are the
+// pops one by one, with the same tours, checklist order and counts; the
+// nodes after it stay pending and are evaluated again.  A node's candidates
+// worth a gain (those nearer than its tour neighbour, a prefix of its row
+// for each of the two kinds) are few -- 6.5 per pop of 2 x 20 on the N=1000
+// panel -- so the prefixes of all nodes are packed one per lane:
+//   lanes 2i + kind   node i's neighbour of that kind and its length
+//   all lanes         the prefix lengths of the 2 x kPopNodes segments, by
+//                     one ballot each over the node's row
+//   lane t            the t-th candidate of the concatenated segments
+// Nodes whose segments end past lane 31 wait for the next pass; a first node
+// that fills more than a warp alone (both kinds wide) takes two rounds.
+//
+// Bound by the ant's chain of dependent instructions (one warp issues every
+// ~6 cycles); a pass resolves about two pops for the chain of one.  One GB300,
+// against one pop per pass: one N=100 colony, 64 iterations 8.78 -> 7.46 ms;
+// 256 x 32 ants at N=1000, 320 iterations 151 -> 136 ms; the uneven batch
+// (N 200-1000, 400 iterations) 145 -> 122 ms; 128 x 32 at N=1000-2000, 640
+// iterations 228 -> 205 ms.
+constexpr std::uint32_t kPopNodes = 4;
+
 __device__ __forceinline__ void checklist_two_opt(const AntSmem& s, const int2* xy, const InstanceView& in,
                                                   std::uint32_t n, std::uint32_t lane, Checklist& q,
                                                   unsigned long long cap, AntResult& r, long long& gain_sum,
                                                   std::uint32_t* log, std::uint32_t log_cap) {
     const std::uint32_t w = in.w;
-    LsRow next{n, n, 0};
+    // evaluations stay far below 2^32 (at most 2 w per pop, a few pops per accepted move, n moves)
+    const std::uint32_t limit = cap < 0xffffffffull ? (std::uint32_t)cap : 0xffffffffu;
+    std::uint32_t evaluations = 0;
+    const std::uint32_t kind = lane & 1u;
     while (q.pending > 0 && r.accepted < n) {
-        if (r.evaluations >= cap) { r.limit_reached = 1; break; }
-        const LsRow row = pop_with_row(s, q, n, lane, in, next);
-        const std::uint32_t a = row.node, b = row.b;
-        const int ab = row.ab;
-        const std::uint32_t pa = s.pos[a];
-        const std::uint32_t an = s.tour[pa + 1 == n ? 0 : pa + 1];
-        const std::uint32_t ap = s.tour[pa == 0 ? n - 1 : pa - 1];
-        ++r.processed;
-        const int2 pa_xy = xy[a];
-        const int cur0 = euc2d(pa_xy, xy[an]), cur1 = euc2d(xy[ap], pa_xy);
-        // prefix of candidates that pass the distance test, per kind
-        const bool bad0 = lane < w && (b >= n || !(cur0 > ab));
-        const bool bad1 = lane < w && (b >= n || !(cur1 > ab));
-        const unsigned f0m = __ballot_sync(kFull, bad0), f1m = __ballot_sync(kFull, bad1);
-        const std::uint32_t f0 = f0m ? __ffs(f0m) - 1 : w, f1 = f1m ? __ffs(f1m) - 1 : w;
-        unsigned long long remaining = cap - r.evaluations;
-        const std::uint32_t used0 = remaining < f0 ? (std::uint32_t)remaining : f0;
-        r.evaluations += used0;
-        r.checks += used0 + (used0 < w ? 1 : 0);
-        if (used0 < f0) { r.limit_reached = 1; break; }
-        remaining = cap - r.evaluations;
-        const std::uint32_t used1 = remaining < f1 ? (std::uint32_t)remaining : f1;
-        r.evaluations += used1;
-        r.checks += used1 + (used1 < w ? 1 : 0);
-        if (used1 < f1) { r.limit_reached = 1; break; }
-        // gains
-        int g0 = INT_MIN, g1 = INT_MIN;
-        std::uint32_t nb0 = 0, nb1 = 0;
-        if (lane < used0 || lane < used1) {
-            const std::uint32_t pb = s.pos[b];
-            const int2 bxy = xy[b];
-            if (lane < used0) {
-                nb0 = s.tour[pb + 1 == n ? 0 : pb + 1];
-                g0 = (nb0 == a || b == an) ? 0 : cur0 + euc2d(bxy, xy[nb0]) - ab - euc2d(xy[an], xy[nb0]);
-            }
-            if (lane < used1) {
-                nb1 = s.tour[pb == 0 ? n - 1 : pb - 1];
-                g1 = (nb1 == a || b == ap) ? 0 : cur1 + euc2d(bxy, xy[nb1]) - ab - euc2d(xy[ap], xy[nb1]);
+        if (evaluations >= limit) { r.limit_reached = 1; break; }
+        // lane 2i + kind: node i (the first one again where fewer are pending), its neighbour and edge length
+        const std::uint32_t i = (lane >> 1) & (kPopNodes - 1);
+        const bool live = i < q.pending;
+        std::uint32_t at = live ? q.head + i : q.head;
+        if (at >= n) at -= n;
+        const std::uint32_t a = s.ring[at];
+        std::uint32_t row_b[kPopNodes];
+        int row_ab[kPopNodes];
+#pragma unroll
+        for (std::uint32_t t = 0; t < kPopNodes; ++t) {
+            const std::size_t row = (std::size_t)__shfl_sync(kFull, a, 2 * t) * w + lane;
+            row_b[t] = n;
+            row_ab[t] = INT_MAX;
+            if (lane < w) {
+                row_b[t] = __ldg(in.ls + row);
+                row_ab[t] = __ldg(in.ls_dist + row);
             }
         }
-        const int best = __reduce_max_sync(kFull, g0 > g1 ? g0 : g1);
-        if (best > 0) {
-            const std::uint32_t mine = g0 == best ? lane : g1 == best ? w + lane : 0xffu;
-            const std::uint32_t index = __reduce_min_sync(kFull, mine);
-            const std::uint32_t kind = index >= w, j = kind ? index - w : index;
-            const std::uint32_t bj = __shfl_sync(kFull, b, j);
-            const std::uint32_t nbj = __shfl_sync(kFull, kind ? nb1 : nb0, j);
-            std::uint32_t m0, m1, m2, m3;
-            if (kind == 0) { m0 = an; m1 = nbj; m2 = a; m3 = bj; }
-            else { m0 = a; m1 = bj; m2 = ap; m3 = nbj; }
-            r.moved += flip(s, n, lane, m0, m1);
-            if constexpr (kCompact) {
-#pragma unroll 1
-                for (int t = 0; t < 4; ++t)
-                    r.reactivations += push_absent(s, q, n, t == 0 ? m0 : t == 1 ? m1 : t == 2 ? m2 : m3, lane, log,
-                                                   log_cap);
-            } else {
-                r.reactivations += push_absent(s, q, n, m0, lane, log, log_cap);
-                r.reactivations += push_absent(s, q, n, m1, lane, log, log_cap);
-                r.reactivations += push_absent(s, q, n, m2, lane, log, log_cap);
-                r.reactivations += push_absent(s, q, n, m3, lane, log, log_cap);
+        const std::uint32_t pa = s.pos[a];
+        const std::uint32_t end = s.tour[kind ? (pa == 0 ? n - 1 : pa - 1) : (pa + 1 == n ? 0 : pa + 1)];
+        const int cur = live ? euc2d(xy[a], xy[end]) : -1;
+        // segment ends: off[2i + kind + 1]
+        std::uint32_t off[2 * kPopNodes + 1];
+        off[0] = 0;
+#pragma unroll
+        for (std::uint32_t g = 0; g < 2 * kPopNodes; ++g) {
+            const int c = __shfl_sync(kFull, cur, g);
+            off[g + 1] = off[g] + __popc(__ballot_sync(kFull, c > row_ab[g >> 1] && row_b[g >> 1] < n));
+        }
+        std::uint32_t nodes = 1;
+#pragma unroll
+        for (std::uint32_t t = 2; t <= kPopNodes; ++t)
+            if (off[2 * t] <= 32u) nodes = t;
+        nodes = nodes < q.pending ? nodes : q.pending;
+        std::uint32_t total = off[2];
+#pragma unroll
+        for (std::uint32_t t = 2; t <= kPopNodes; ++t)
+            if (nodes == t) total = off[2 * t];
+        if (total >= limit - evaluations) {
+            // the budget may end here: the first node alone, cut where the budget ends
+            nodes = 1;
+            total = off[2];
+            const std::uint32_t left = limit - evaluations, f0 = off[1], f1 = off[2] - off[1];
+            const bool cut0 = left < f0, cut1 = !cut0 && left - f0 < f1;
+            if (cut0 || cut1) {
+                evaluations += left;
+                r.checks += left + 1 + (cut1 && f0 < w ? 1 : 0);
+                ++r.processed;
+                r.limit_reached = 1;
+                break;
             }
+        }
+        // lane t: the t-th candidate of the segments
+        int gain = 0;
+        std::uint32_t best_t = 0, best_seg = 0, best_b = 0, best_nb = 0;
+        for (std::uint32_t base = 0; base < total; base += 32) {
+            const std::uint32_t t = base + lane;
+            const bool on = t < total;
+            // the segment of t, by halving
+            const bool h2 = t >= off[4];
+            const std::uint32_t e1 = h2 ? off[6] : off[2];
+            const bool h1 = t >= e1;
+            const std::uint32_t e0 = h2 ? (h1 ? off[7] : off[5]) : (h1 ? off[3] : off[1]);
+            const bool h0 = t >= e0;
+            const std::uint32_t seg = on ? (h2 ? 4u : 0u) + (h1 ? 2u : 0u) + (h0 ? 1u : 0u) : 0u;
+            const std::uint32_t j = on ? t - (h0 ? e0 : h1 ? e1 : h2 ? off[4] : 0u) : 0u;
+            const std::uint32_t node = __shfl_sync(kFull, a, seg), close = __shfl_sync(kFull, end, seg);
+            const int edge = __shfl_sync(kFull, cur, seg);
+            std::uint32_t b = __shfl_sync(kFull, row_b[0], j);
+            int ab = __shfl_sync(kFull, row_ab[0], j);
+#pragma unroll
+            for (std::uint32_t x = 1; x < kPopNodes; ++x) {
+                const std::uint32_t bx = __shfl_sync(kFull, row_b[x], j);
+                const int abx = __shfl_sync(kFull, row_ab[x], j);
+                if ((seg >> 1) == x) { b = bx; ab = abx; }
+            }
+            if (on) {
+                const std::uint32_t pb = s.pos[b];
+                const std::uint32_t nb = s.tour[seg & 1u ? (pb == 0 ? n - 1 : pb - 1) : (pb + 1 == n ? 0 : pb + 1)];
+                const int2 nxy = xy[nb];
+                const int g = nb == node || b == close ? 0 : edge - ab + euc2d(xy[b], nxy) - euc2d(xy[close], nxy);
+                if (g > gain) { gain = g; best_t = t; best_seg = seg; best_b = b; best_nb = nb; }
+            }
+        }
+        const unsigned improving = __ballot_sync(kFull, gain > 0);
+        // the pops: up to the first node with a move, else all
+        std::uint32_t popped = nodes;
+        if (improving) popped = (__shfl_sync(kFull, best_seg, __ffs(improving) - 1) >> 1) + 1;
+        std::uint32_t done = off[2];
+#pragma unroll
+        for (std::uint32_t t = 2; t <= kPopNodes; ++t)
+            if (popped == t) done = off[2 * t];
+        evaluations += done;
+        r.processed += popped;
+        r.checks += done;
+#pragma unroll
+        for (std::uint32_t g = 0; g < 2 * kPopNodes; ++g)
+            r.checks += (g >> 1) < popped && off[g + 1] - off[g] < w ? 1 : 0;
+        q.head += popped;
+        if (q.head >= n) q.head -= n;
+        q.pending -= popped;
+        for (std::uint32_t t = 0; t < popped; ++t) {   // one at a time: nodes may share a word
+            if (lane == 2 * t) s.queued[a >> 5] &= ~(1u << (a & 31u));
+            __syncwarp();
+        }
+        if (improving) {
+            const bool mine = gain > 0 && (best_seg >> 1) + 1 == popped;
+            const int best = __reduce_max_sync(kFull, mine ? gain : 0);
+            const std::uint32_t first = __reduce_min_sync(kFull, mine && gain == best ? best_t : 0xffu);
+            const std::uint32_t src = first & 31u, seg = __shfl_sync(kFull, best_seg, src);
+            const std::uint32_t bj = __shfl_sync(kFull, best_b, src), nbj = __shfl_sync(kFull, best_nb, src);
+            const std::uint32_t node = __shfl_sync(kFull, a, seg), close = __shfl_sync(kFull, end, seg);
+            // reversed between m0 and m1; all four ends become pending, in this order
+            const bool back = seg & 1u;
+            const std::uint32_t m0 = back ? node : close, m1 = back ? bj : nbj;
+            const std::uint32_t m2 = back ? close : node, m3 = back ? nbj : bj;
+            r.moved += flip(s, n, lane, m0, m1);
+            r.reactivations += push_lanes(s, q, n, lane == 0 ? m0 : lane == 1 ? m1 : lane == 2 ? m2 : m3, lane < 4,
+                                          lane, log, log_cap);
             ++r.accepted;
             gain_sum -= best;
         }
-        __syncwarp();
     }
+    r.evaluations += evaluations;
 }
 
 // Checklist local search with first-improvement 2-opt then Or-opt (segments
