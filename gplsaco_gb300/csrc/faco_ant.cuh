@@ -380,85 +380,60 @@ struct RelocationRun {
 // every lane of the chosen hypothesis was taken (the walk may go on).
 __device__ __forceinline__ bool on_segment(int lo, int hi, int q) { return q >= lo && q <= hi; }
 
-// The roulette of one lane's step in follow_batch: the candidates of `row`
-// still open to the walk (unvisited, and for a relocation run not on the
-// run's segment), their FP32 weights summed serially in candidate order,
-// and the first prefix at or above uf * total; -1 when that prefix lies
-// within the decision margin (the one-step path decides) or no candidate is
-// open.  The dense variants unroll both loops by two; the others leave them
-// to the compiler.  The loops are written out twice because any rewrite of
-// the shared body (a lambda, a helper per candidate) changed the compiler's
-// code for the latency-tuned variants.  Both run the same sums in the same
-// order.
-template <bool kDense>
-__device__ __forceinline__ int follow_roulette(const AntSmem& s, const node_t* row, const float* prow,
-                                               std::uint32_t n, std::uint32_t k, std::uint32_t rel, std::uint32_t t0,
-                                               bool identity, int lo, int hi, float uf) {
-    unsigned avail = 0;
-    float tot = 0.0f;
-    if constexpr (kDense) {
-#pragma unroll 2
-        for (std::uint32_t j = 0; j < k; ++j) {
-            const std::uint32_t x = __ldg(row + j);
-            const float w = __ldg(prow + j);
-            bool a = x < n && !test_bit(s.visited, x);
-            if (a && rel) {
-                const std::uint32_t px = s.pos[x];
-                const std::uint32_t dx = px >= t0 ? px - t0 : px + n - t0;   // tour positions after the start
-                a = identity ? !(dx >= 1 && dx <= rel) : !on_segment(lo, hi, (int)px);
+// Whether one lane's step in follow_batch draws `sel`: the candidates of
+// `row` still open to the walk (unvisited, and neither on the identity walk
+// nor on the relocation run taken by the earlier lanes), their FP32 weights
+// summed serially in candidate order.  The first prefix at or above uf *
+// total is sel's own, by the decision margin on both sides, exactly when the
+// prefix before sel is certainly below the threshold and the one with sel
+// certainly above it; so one pass over the row decides, with the total and
+// those two prefixes.  False where the margin leaves it open (the one-step
+// path then decides).  Rows of a multiple of four candidates are read four
+// at a time (8 + 16 bytes), one group ahead of the sums.
+__device__ __forceinline__ bool follow_takes(const AntSmem& s, const node_t* row, const float* prow, std::uint32_t n,
+                                             std::uint32_t k, std::uint32_t sel, std::uint32_t rel, std::uint32_t t0,
+                                             bool identity, int lo, int hi, float uf) {
+    float total = 0.0f, before = 0.0f, upto = -1.0f;
+    bool any = false, earlier = false;
+    // (adding zero for a closed candidate leaves the sum as it is)
+    const auto add = [&](std::uint32_t x, float weight) {
+        const std::uint32_t px = s.pos[x];
+        const std::uint32_t dx = px >= t0 ? px - t0 : px + n - t0;   // tour positions after the start
+        const bool on_path = identity ? dx - 1u < rel : on_segment(lo, hi, (int)px);
+        const bool open = !(test_bit(s.visited, x) | (rel && on_path)), mine = open && x == sel;
+        before = mine ? total : before;
+        earlier = mine ? any : earlier;
+        total += open ? weight : 0.0f;
+        upto = mine ? total : upto;
+        any |= open;
+    };
+    if ((k & 3u) == 0) {
+        const uint2* rows = reinterpret_cast<const uint2*>(row);
+        const float4* weights = reinterpret_cast<const float4*>(prow);
+        uint2 x = __ldg(rows);
+        float4 p = __ldg(weights);
+#pragma unroll 1
+        for (std::uint32_t g = 1; g <= k / 4; ++g) {
+            const uint2 xg = x;
+            const float4 pg = p;
+            if (g < k / 4) {
+                x = __ldg(rows + g);
+                p = __ldg(weights + g);
             }
-            if (a) {
-                avail |= 1u << j;
-                tot += w;
-            }
+            add(xg.x & 0xffffu, pg.x);
+            add(xg.x >> 16, pg.y);
+            add(xg.y & 0xffffu, pg.z);
+            add(xg.y >> 16, pg.w);
         }
     } else {
-        for (std::uint32_t j = 0; j < k; ++j) {
-            const std::uint32_t x = __ldg(row + j);
-            const float w = __ldg(prow + j);
-            bool a = x < n && !test_bit(s.visited, x);
-            if (a && rel) {
-                const std::uint32_t px = s.pos[x];
-                const std::uint32_t dx = px >= t0 ? px - t0 : px + n - t0;   // tour positions after the start
-                a = identity ? !(dx >= 1 && dx <= rel) : !on_segment(lo, hi, (int)px);
-            }
-            if (a) {
-                avail |= 1u << j;
-                tot += w;
-            }
-        }
+#pragma unroll 1
+        for (std::uint32_t j = 0; j < k; ++j) add(__ldg(row + j), __ldg(prow + j));
     }
-    int choice = -1;
-    if (avail && tot >= 0x1p-100f) {
-        const float thr = uf * tot, delta = tot * 0x1p-17f;
-        float prefix = 0.0f;
-        if constexpr (kDense) {
-#pragma unroll 2
-            for (std::uint32_t j = 0; j < k; ++j) {
-                if (!((avail >> j) & 1u)) continue;
-                prefix += __ldg(prow + j);
-                const float diff = prefix - thr;
-                if (diff >= -delta) {
-                    if (diff > delta) choice = (int)j;
-                    break;
-                }
-            }
-        } else {
-            for (std::uint32_t j = 0; j < k; ++j) {
-                if (!((avail >> j) & 1u)) continue;
-                prefix += __ldg(prow + j);
-                const float diff = prefix - thr;
-                if (diff >= -delta) {
-                    if (diff > delta) choice = (int)j;
-                    break;
-                }
-            }
-        }
-    }
-    return choice;
+    if (!(total >= 0x1p-100f)) return false;
+    const float threshold = uf * total, delta = total * 0x1p-17f;
+    return (!earlier || before - threshold < -delta) && upto - threshold > delta;
 }
 
-template <bool kDense>
 __device__ inline std::uint32_t follow_batch(const AntSmem& s, const int2* xy, const InstanceView& in,
                                              const float* products, const std::uint32_t* parent_nbr, std::uint32_t n,
                                              std::uint32_t lane, unsigned long long key, std::uint32_t batch,
@@ -542,8 +517,7 @@ __device__ inline std::uint32_t follow_batch(const AntSmem& s, const int2* xy, c
     if (ok) {
         const node_t* row = in.primary + (size_t)cur * k;
         const float* prow = products + (size_t)cur * k;
-        const int choice = follow_roulette<kDense>(s, row, prow, n, k, rel, t0, identity, lo, hi, uf);
-        ok = choice >= 0 && __ldg(row + choice) == sel;
+        ok = follow_takes(s, row, prow, n, k, sel, rel, t0, identity, lo, hi, uf);
     }
     // the leading run of taken steps
     const unsigned okm = __ballot_sync(kFull, ok);

@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
             if (++guard > loop_cap) { if (lane == 0) atomicOr(L.error, kErrLoopCap); break; }
             if (kFollow && follow) {
                 bool full = false;
-                const std::uint32_t f = follow_batch<kDense>(s, xy, in, products, parent_nbr, n, lane, key, batch,
+                const std::uint32_t f = follow_batch(s, xy, in, products, parent_nbr, n, lane, key, batch,
                                                              ant, current, r, cost, run, draw_base, draw_hi, draw_lo,
                                                              full);
                 follow = full;
