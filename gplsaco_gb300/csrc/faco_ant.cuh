@@ -42,11 +42,8 @@ enum AntMode : int {
                             // coordinates read from global (large instances)
     kModeEngineFollow = 5,        // kModeEngine with batched parent-following steps (follow_batch)
     kModeEngineGlobalFollow = 6,  // kModeEngineGlobal with batched parent-following steps
-    // kModeEngineFollow compiled for panels beyond one wave of the GPU: the
-    // same arithmetic, the batch's roulette loops unrolled by two (72
-    // registers against 79: one more block per SM) where mode 5 favours one
-    // ant's latency.  The global-workspace variant has no such build: the
-    // same unrolling leaves it at 80 registers.
+    // kModeEngineFollow with fewer registers, for panels beyond one wave of
+    // the GPU (ant_blocks_per_sm)
     kModeEngineFollowDense = 7,
 };
 
@@ -84,6 +81,8 @@ struct AntLaunch {
     std::uint32_t n_max;          // smem layout size
     unsigned long long ls_limit;
     std::uint32_t ls_mode;
+    std::uint32_t batch_from;     // batched variants: colonies whose ants walked at least this many steps
+                                  // in their last iteration (ColonyView::walk; 0: all) use the batches
     // diagnostic modes: tasks on instance 0
     std::uint32_t tasks;
     const node_t* task_tours;        // [tasks][n]

@@ -186,6 +186,7 @@ struct ColonyView {
     node_t* archive;               // [2 sides][4 slots][tour, positions][n_pad]
     unsigned long long* ant_ids;   // [ants][2] fingerprints of the batch's tours
     std::uint32_t* ant_p0;         // [ants] position of node 0 in each tour
+    std::uint32_t* walk;           // construction steps per ant of the last iteration (null: not kept)
 };
 
 struct TraceRow {

@@ -17,7 +17,6 @@
 #include <map>
 #include <memory>
 #include <mutex>
-#include <optional>
 #include <stdexcept>
 #include <string>
 #include <thread>
@@ -35,20 +34,16 @@ thread_local std::string g_error;
 
 // Iterations captured per CUDA graph (replayed until the budget is spent).
 constexpr std::uint32_t kGraphIterations = 16;
-// Batched steps chosen per stretch of iterations (FACO_FOLLOW_AUTO on panels
-// beyond one wave of ant warps): every kAdaptIterations iterations the
-// colonies' step counters are read back, and the following replays take the
-// batched-step graph once the stretch averaged at least kBatchOnSteps
-// construction steps per ant and iteration, the one-step graph again below
-// kBatchOffSteps.  Measured on the N=1000 throughput panel: batches lose up
-// to 1.9x on the short walks of early iterations (11-30 steps), break even
-// near 70 and win 19-26 % from 110 steps on.
-// With the global-memory ant workspace (large instances) the crossover is
-// later: on the large clustered panel (N 5,750-9,650) batches lose up to 17 %
-// below 50 steps and win 6-11 % from 150 on.
-constexpr std::uint32_t kAdaptIterations = 32;   // 64 switched one stretch later: 3 % slower on iterations 0-320
-constexpr double kBatchOnSteps = 72.0, kBatchOffSteps = 60.0;
-constexpr double kBatchOnStepsGlobal = 96.0, kBatchOffStepsGlobal = 80.0;
+// FACO_FOLLOW_AUTO: a colony takes parent-following steps in batches from
+// this many construction steps per ant on, as walked in its last iteration
+// (the ant kernel reads it); below, the batches' setup costs more than the
+// few steps they take at once.  Measured in us per iteration, one at a time /
+// in batches: the uneven batch (4,096 ant warps) 179 / 211 at 23 steps, 224 /
+// 226 at 31, 297 / 251 at 44; 256 x 32 ants at N=1000 340 / 416 at 33 steps,
+// 438 / 448 at 51, 601 / 500 at 80; the large panel in the global-memory
+// workspace (2-opt) 1814 / 1857 at 54, 2195 / 1994 at 80.  Moving a line by a
+// fifth either way changes a run by less than 1 %.
+constexpr std::uint32_t kBatchFromOneWave = 30, kBatchFromFull = 48, kBatchFromGlobal = 60;
 // Automatic chain count: one chain per kColoniesPerChain colonies, at most kMaxChains.
 // Trail updates of more than 2 x kTrailCellsPerBlock entries per colony run in
 // colony_trails_kernel, one block per kTrailCellsPerBlock entries (at most
@@ -279,6 +274,7 @@ struct faco_engine {
     DeviceBuffer<long long> ant_costs, ant_ccosts;
     DeviceBuffer<faco::Program> programs;
     DeviceBuffer<unsigned> ant_counts, error;
+    DeviceBuffer<std::uint32_t> walks;          // per colony: construction steps per ant of its last iteration
     DeviceBuffer<faco::ColonyState> states;
     DeviceBuffer<faco::ColonyView> colonies;
     DeviceBuffer<uint2> work;
@@ -340,16 +336,8 @@ struct faco_engine {
         faco::AntLaunch L{};
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
-        // batched steps chosen per stretch of iterations: the batched-step
-        // graph beside the one-step one, the variant of the next replays and
-        // the step counters at the last reading
-        bool adaptive = false, batched = false;
-        double batch_on = kBatchOnSteps, batch_off = kBatchOffSteps;
-        cudaGraph_t graph_batched = nullptr;
-        cudaGraphExec_t exec_batched = nullptr;
-        unsigned long long steps_seen = 0;
-        std::uint32_t done_seen = 0;
-        bool rebase = false;                    // the next reading only sets the baseline (restored runs)
+        bool full = false;                      // more ant warps than one wave of the GPU
+        std::uint32_t batch_from = 0;           // AntLaunch::batch_from
     } eval;
     std::vector<cudaStream_t> branch_streams;
     std::vector<cudaEvent_t> branch_events;   // [0] fork, [1 + i] join of branch i
@@ -360,8 +348,6 @@ struct faco_engine {
     ~faco_engine() {
         if (eval.exec) cudaGraphExecDestroy(eval.exec);
         if (eval.graph) cudaGraphDestroy(eval.graph);
-        if (eval.exec_batched) cudaGraphExecDestroy(eval.exec_batched);
-        if (eval.graph_batched) cudaGraphDestroy(eval.graph_batched);
         for (auto st : branch_streams) cudaStreamDestroy(st);
         for (auto ev : branch_events) cudaEventDestroy(ev);
         if (stream) {
@@ -614,12 +600,8 @@ namespace {
 void destroy_graph(faco_engine* e) {
     if (e->eval.exec) cudaGraphExecDestroy(e->eval.exec);
     if (e->eval.graph) cudaGraphDestroy(e->eval.graph);
-    if (e->eval.exec_batched) cudaGraphExecDestroy(e->eval.exec_batched);
-    if (e->eval.graph_batched) cudaGraphDestroy(e->eval.graph_batched);
     e->eval.exec = nullptr;
     e->eval.graph = nullptr;
-    e->eval.exec_batched = nullptr;
-    e->eval.graph_batched = nullptr;
 }
 
 // All ant launches of one iteration: class 0 on `st`, the others on branch
@@ -712,7 +694,9 @@ void enqueue_iterations(faco_engine* e, cudaStream_t st, std::uint32_t iteration
 // The evaluation's graph: kGraphIterations iterations, replayed.  A failed
 // enqueue ends the capture (discarding the partial graph) before the error
 // propagates, so the stream is usable again.
-void capture_one(faco_engine* e, cudaStream_t st, cudaGraph_t& graph, cudaGraphExec_t& exec) {
+void capture_graph(faco_engine* e, cudaStream_t st) {
+    destroy_graph(e);
+    auto& v = e->eval;
     cuda_check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
     try {
         enqueue_iterations(e, st, kGraphIterations);
@@ -722,48 +706,10 @@ void capture_one(faco_engine* e, cudaStream_t st, cudaGraph_t& graph, cudaGraphE
         cudaGetLastError();
         throw;
     }
-    cuda_check(cudaStreamEndCapture(st, &graph), "end capture");
-    cuda_check(cudaGraphInstantiate(&exec, graph, 0), "graph instantiate");
+    cuda_check(cudaStreamEndCapture(st, &v.graph), "end capture");
+    cuda_check(cudaGraphInstantiate(&v.exec, v.graph, 0), "graph instantiate");
     // upload now, so that the first replay costs what every other one does
-    cuda_check(cudaGraphUpload(exec, st), "graph upload");
-}
-
-// While alive, every class of an adaptive evaluation launches its
-// batched-step variant (the build for panels beyond one wave); the
-// one-step modes come back when it ends, an exception included.
-class BatchedModes {
-  public:
-    explicit BatchedModes(faco_engine::EvalState& v) : v_(v) {
-        for (auto& cl : v_.classes) {
-            modes_.push_back(cl.mode);
-            cl.mode = faco::with_follow(cl.mode, true);
-        }
-    }
-    ~BatchedModes() {
-        for (std::size_t i = 0; i < modes_.size(); ++i) v_.classes[i].mode = modes_[i];
-    }
-    BatchedModes(const BatchedModes&) = delete;
-    BatchedModes& operator=(const BatchedModes&) = delete;
-
-  private:
-    faco_engine::EvalState& v_;
-    std::vector<int> modes_;
-};
-
-void capture_graph(faco_engine* e, cudaStream_t st) {
-    auto& v = e->eval;
-    destroy_graph(e);
-    capture_one(e, st, v.graph, v.exec);
-    if (v.adaptive) {
-        // the same iterations with every class's batched-step variant
-        BatchedModes batched(v);
-        capture_one(e, st, v.graph_batched, v.exec_batched);
-    }
-    // a fresh evaluation starts with every counter at zero
-    v.batched = false;
-    v.steps_seen = 0;
-    v.done_seen = 0;
-    v.rebase = false;
+    cuda_check(cudaGraphUpload(v.exec, st), "graph upload");
 }
 
 // Kernel variant of a size class: the global-memory workspace (tour and
@@ -803,6 +749,13 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
             for (std::uint32_t a = 0; a < A; a += warps) jobs.push_back(make_uint2(col, a));
         return jobs;
     };
+    // batched parent-following steps (the same results): always on request,
+    // else per colony from its walk length; panels with more ant warps than
+    // one wave of the GPU run the build that favours throughput over one
+    // ant's latency
+    v.full = static_cast<std::uint64_t>(v.count) * A > 32ull * static_cast<std::uint64_t>(e->sm_count);
+    v.follow = c.follow != FACO_FOLLOW_OFF;
+    v.batch_from = c.follow == FACO_FOLLOW_ON ? 0u : v.full ? kBatchFromFull : kBatchFromOneWave;
     bool need_workspace = false;
     for (const auto& cl : v.classes) need_workspace = need_workspace || may_use_global(c, cl.n_max);
     if (need_workspace) e->ant_workspace.resize(2 * e->ant_tours.size());
@@ -823,6 +776,7 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
         L.n_max = n_max;
         L.workspace = need_workspace ? e->ant_workspace.get() : nullptr;
         L.ant_tours_base = e->ant_tours.get();
+        L.batch_from = v.batch_from;
         return L;
     };
     if (c.autotune) {
@@ -835,7 +789,8 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
                                       (static_cast<std::uint64_t>(cl.n_max) << 40) ^
                                       (static_cast<std::uint64_t>(A) << 24) ^
                                       (static_cast<std::uint64_t>(members[i].size()) << 4) ^
-                                      (static_cast<std::uint64_t>(c.workspace) << 2) ^ c.ls_mode;
+                                      (static_cast<std::uint64_t>(c.workspace) << 2) ^
+                                      (static_cast<std::uint64_t>(v.full) << 1) ^ c.ls_mode;
             const auto hit = e->tuned_warps.find(key);
             if (hit != e->tuned_warps.end()) {
                 cl.warps = hit->second.first;
@@ -844,6 +799,7 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
             }
             float best_ms = 0.0f;
             for (const int mode : {static_cast<int>(faco::kModeEngine), static_cast<int>(faco::kModeEngineGlobal)}) {
+                const int timed = v.follow ? faco::with_follow(mode, v.full) : mode;   // the variant that will run
                 if (mode == faco::kModeEngine && !may_use_shared(c, cl.n_max)) continue;
                 if (mode == faco::kModeEngineGlobal && !may_use_global(c, cl.n_max)) continue;
                 for (std::uint32_t w = 1; w <= faco::kMaxWarpsPerBlock && w <= A; w *= 2) {
@@ -852,11 +808,11 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
                     const auto jobs = jobs_for(members[i], w);
                     e->work.upload(jobs, s);
                     const faco::AntLaunch L = launch_of(0, w, cl.n_max);
-                    cuda_check(faco::prepare_ant_kernel(mode, smem), "attribute");
+                    cuda_check(faco::prepare_ant_kernel(timed, smem), "attribute");
                     float ms = 0.0f;
                     for (int rep = 0; rep < 3; ++rep) {
                         cuda_check(cudaEventRecord(t0, s), "event");
-                        cuda_check(faco::launch_ant_kernel(mode, L, static_cast<std::uint32_t>(jobs.size()), w, smem, s),
+                        cuda_check(faco::launch_ant_kernel(timed, L, static_cast<std::uint32_t>(jobs.size()), w, smem, s),
                                    "tuning launch");
                         cuda_check(cudaEventRecord(t1, s), "event");
                         cuda_check(cudaEventSynchronize(t1), "tuning");
@@ -916,23 +872,11 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
         else e->chain_colonies.upload(list, s);
     }
     e->work.upload(all, s);
-    // batched parent-following steps (the same results): on request, or
-    // when every ant warp of the evaluation fits in one wave of the GPU
-    const std::uint64_t ant_warps = static_cast<std::uint64_t>(v.count) * A;
-    const bool one_wave = ant_warps <= 32ull * static_cast<std::uint64_t>(e->sm_count);
-    v.follow = c.follow == FACO_FOLLOW_ON || (c.follow == FACO_FOLLOW_AUTO && one_wave);
-    // beyond one wave the automatic choice is made per stretch of iterations
-    // from the walk length (step_evaluation), with the later crossover of
-    // the global-memory workspace when a class uses it
-    bool any_global = false;
-    for (const auto& cl : v.classes) any_global = any_global || faco::global_mode(cl.mode);
-    v.adaptive = c.follow == FACO_FOLLOW_AUTO && !one_wave;
-    v.batch_on = any_global ? kBatchOnStepsGlobal : kBatchOnSteps;
-    v.batch_off = any_global ? kBatchOffStepsGlobal : kBatchOffSteps;
-    // (beyond one wave, the batched build that favours throughput over one
-    // ant's latency)
+    if (v.batch_from)
+        for (const auto& cl : v.classes)
+            if (faco::global_mode(cl.mode)) v.batch_from = kBatchFromGlobal;
     if (v.follow)
-        for (auto& cl : v.classes) cl.mode = faco::with_follow(cl.mode, !one_wave);
+        for (auto& cl : v.classes) cl.mode = faco::with_follow(cl.mode, v.full);
     // the dynamic shared-memory limit is a property of each kernel variant,
     // shared by every class that uses it: it must admit the largest one
     std::map<int, std::uint32_t> smem_max;
@@ -942,11 +886,8 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
         m = std::max(m, cl.smem);
     }
     for (auto& ch : v.chains) ch.L = launch_of(ch.first_job, v.classes[ch.cls].warps, v.classes[ch.cls].n_max);
-    for (const auto& [mode, smem] : smem_max) {
+    for (const auto& [mode, smem] : smem_max)
         if (smem) cuda_check(faco::prepare_ant_kernel(mode, smem), "cudaFuncSetAttribute");
-        if (smem && v.adaptive)
-            cuda_check(faco::prepare_ant_kernel(faco::with_follow(mode, true), smem), "cudaFuncSetAttribute");
-    }
 }
 
 // Controller programs of a GP-controlled evaluation (null: plain FACO).
@@ -1086,6 +1027,7 @@ void begin_evaluation(faco_engine* e, const uint64_t* keys, const uint64_t* seed
         e->decision_actions.resize(slots);
     }
     e->ant_counts.resize(3ull * A * count);
+    e->walks.resize(count);
     e->states.resize(count);
     std::size_t tau_off = 0, node_off = 0, ant_off = 0;
     for (std::uint32_t c = 0; c < count; ++c) {
@@ -1109,6 +1051,7 @@ void begin_evaluation(faco_engine* e, const uint64_t* keys, const uint64_t* seed
         cv.action_mask = control.action_mask;
         cv.controller_kind = control.programs ? control.kinds[c / replicas] : 0u;
         cv.ant_counts = e->ant_counts.get() + 3ull * c * A;
+        cv.walk = e->walks.get() + c;
         if (spec == 2) {
             cv.control = e->ref_controls.get() + c;
             cv.archive = e->archives.get() + 16ull * node_off;
@@ -1204,52 +1147,17 @@ void begin_evaluation(faco_engine* e, const uint64_t* keys, const uint64_t* seed
     v.active = true;
 }
 
-// The batched or one-step graph for the next replays, from the average
-// construction steps per ant and iteration since the last reading (the
-// colonies' counters, read after the stream drains: one synchronisation per
-// kAdaptIterations iterations).  Results do not depend on the choice.
-void choose_variant(faco_engine* e) {
-    auto& v = e->eval;
-    std::vector<faco::ColonyState> states(v.count);
-    e->states.download(states.data(), v.count, e->stream);
-    cuda_check(cudaStreamSynchronize(e->stream), "step counters");
-    unsigned long long steps = 0;
-    for (const auto& st : states) steps += st.construction_steps;
-    if (!v.rebase && v.done > v.done_seen && steps >= v.steps_seen) {
-        const double per_ant = static_cast<double>(steps - v.steps_seen) /
-                               (static_cast<double>(v.done - v.done_seen) * v.count * std::max(1u, v.L.ants));
-        if (!v.batched && per_ant >= v.batch_on) v.batched = true;
-        else if (v.batched && per_ant < v.batch_off) v.batched = false;
-    }
-    v.steps_seen = steps;
-    v.done_seen = v.done;
-    v.rebase = false;
-}
-
 void step_evaluation(faco_engine* e, std::uint32_t iterations) {
     auto& v = e->eval;
     require(v.active, "no active evaluation");
-    const auto adapt = [&] {
-        if (v.adaptive && (v.rebase || v.done >= v.done_seen + kAdaptIterations)) choose_variant(e);
-    };
-    std::uint32_t left = iterations;
-    while (left >= kGraphIterations) {
-        adapt();
-        cuda_check(cudaGraphLaunch(v.adaptive && v.batched ? v.exec_batched : v.exec, e->stream), "graph launch");
-        left -= kGraphIterations;
-        v.done += kGraphIterations;
+    for (std::uint32_t left = iterations; left > 0;) {
+        const std::uint32_t now = std::min(left, kGraphIterations);
+        // the rest that fills no graph as direct launches
+        if (now == kGraphIterations) cuda_check(cudaGraphLaunch(v.exec, e->stream), "graph launch");
+        else enqueue_iterations(e, e->stream, now);
+        left -= now;
+        v.done += now;
     }
-    // the rest as direct launches, of the same variant the graphs would run
-    if (left) {
-        adapt();
-        if (v.adaptive && v.batched) {
-            BatchedModes batched(v);
-            enqueue_iterations(e, e->stream, left);
-        } else {
-            enqueue_iterations(e, e->stream, left);
-        }
-    }
-    v.done += left;
 }
 
 void finish_evaluation(faco_engine* e, faco_outputs* out, std::uint32_t dimension) {
@@ -1621,8 +1529,6 @@ int faco_restore(faco_engine* e, const void* buffer, uint64_t bytes, uint32_t tr
             }
             cuda_check(cudaStreamSynchronize(s), "snapshot upload");
             v.done = h.done;
-            v.done_seen = v.done;   // the restored counters run from iteration 0: rebase first
-            v.rebase = true;
         } catch (...) {
             v.active = false;
             destroy_graph(e);
@@ -1662,11 +1568,6 @@ int faco_step_timed(faco_engine* e, uint32_t iterations, double* ant_ms, double*
         std::vector<cudaEvent_t> ev(3 * iterations);
         for (auto& x : ev) cuda_check(cudaEventCreate(&x), "event");
         for (std::uint32_t i = 0; i < iterations; ++i) {
-            // the variant step_evaluation would run (its check falls between
-            // iterations, outside the timed kernels)
-            if (v.adaptive && (v.rebase || v.done >= v.done_seen + kAdaptIterations)) choose_variant(e);
-            std::optional<BatchedModes> batched;
-            if (v.adaptive && v.batched) batched.emplace(v);
             cuda_check(cudaEventRecord(ev[3 * i], s), "event");
             enqueue_ants(e, s);
             cuda_check(cudaEventRecord(ev[3 * i + 1], s), "event");
@@ -1701,7 +1602,7 @@ int faco_get_launch_plan(faco_engine* e, faco_launch_plan* plan) {
         plan->chains = chains;
         plan->graph_iterations = kGraphIterations;
         plan->launches_per_iteration = chains ? chains * (1 + per_update) : plan->size_classes + per_update;
-        plan->follow = v.adaptive ? 2u : v.follow ? 1u : 0u;
+        plan->follow = !v.follow ? 0u : v.full && v.batch_from ? 2u : 1u;
     });
 }
 

@@ -48,10 +48,12 @@ __device__ __forceinline__ void load_parent(const AntSmem& s, const node_t* pare
     }
 }
 
+// the variant's own budget, inside the kernel template
+#define kAntBlocksPerSM (ant_blocks_per_sm(MODE))
+
 template <int MODE>
 __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_kernel(const AntLaunch L) {
-    constexpr bool kEngine = engine_mode(MODE), kGlobalWs = global_mode(MODE), kFollow = follow_mode(MODE),
-                   kDense = dense_mode(MODE);
+    constexpr bool kEngine = engine_mode(MODE), kGlobalWs = global_mode(MODE), kFollow = follow_mode(MODE);
     extern __shared__ __align__(16) unsigned char smem[];
     const std::uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     std::uint32_t colony = 0, ant = 0, task = 0;
@@ -162,8 +164,10 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
         RelocationRun run;
         // steps along the parent tour are taken in batches (follow_batch)
         // until a batch stops short of its lanes; the step it stopped at is
-        // taken alone, then batches resume
-        bool follow = true;
+        // taken alone, then batches resume.  A colony whose walks are short
+        // takes every step alone: the batches' setup is lost on them
+        const bool batches = kFollow && (L.batch_from == 0 || *cv.walk >= L.batch_from);
+        bool follow = batches;
         while (r.mne < target && r.steps + 1 < n) {
             if (++guard > loop_cap) { if (lane == 0) atomicOr(L.error, kErrLoopCap); break; }
             if (kFollow && follow) {
@@ -174,7 +178,7 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
                 follow = full;
                 if (f) continue;
             }
-            follow = true;
+            follow = batches;
             const std::uint32_t step = r.steps + 1;
             if (kEngine && step - draw_base >= 32u) {
                 draw_base = step;
@@ -1329,6 +1333,7 @@ __global__ void colony_init_kernel(const InstanceView* instances, const ColonyVi
         st.epoch_cost = st.global_cost = st.parent_cost = st.iteration_best_cost = in.initial_cost;
         trail_limits(in.initial_cost, P.retention, P.p_root, k, st.tau_min, st.tau_max);
         st.default_trail = st.tau_max;
+        *cv.walk = 0;
         st.mne_target = P.mne_target;
         st.action = -1;
         st.region = 4;
@@ -1468,6 +1473,7 @@ __global__ void __launch_bounds__(256) colony_update_kernel(const InstanceView* 
         st.construction_steps += steps;
         st.ls_evaluations += evals;
         st.reversed_elements += moved;
+        *cv.walk = (std::uint32_t)(steps / A);
         st.default_trail = fmaxf(st.tau_min, st.default_trail * P.retention_f);
         s_st = st;
         s_best = ib; s_improve_epoch = ie; s_improve_global = ig; s_from_epoch = from_epoch;

@@ -62,16 +62,14 @@ typedef struct faco_settings {
                         time, one lane per step; results do not depend on it */
 } faco_settings;
 
-/* Batched parent-following steps: AUTO uses them always when the
- * evaluation's ant warps fit in one wave of the GPU (at most 32 per SM),
- * where an iteration lasts as long as its longest walk.  On fuller panels
- * AUTO chooses every 32 iterations from the walk length of the last 32:
- * batches from 72 construction steps per ant and iteration on, steps one at
- * a time again below 60 (96 and 80 with the global-memory ant workspace of
- * large instances); short walks take more instructions in batches than one
- * at a time.  Beyond one wave the batches run a build of the same steps
- * tuned for throughput (fewer registers per thread, more warps per SM)
- * rather than for one ant's latency. */
+/* Batched parent-following steps: AUTO uses them for the colonies whose ants
+ * walked far in their last iteration, from 30 construction steps per ant on
+ * where the evaluation's ant warps fit in one wave of the GPU (at most 32 per
+ * SM), from 48 on fuller panels and from 60 with the global-memory ant
+ * workspace of large instances: short walks take more instructions in batches
+ * than one at a time.  ON uses them always.  Beyond one wave the ants run a
+ * build of the same steps tuned for throughput (fewer registers per thread,
+ * more warps per SM) rather than for one ant's latency. */
 enum { FACO_FOLLOW_AUTO = 0, FACO_FOLLOW_OFF = 1, FACO_FOLLOW_ON = 2 };
 
 void faco_default_settings(faco_settings* s);
@@ -256,8 +254,9 @@ typedef struct faco_launch_plan {
     uint32_t chains;
     uint32_t graph_iterations;
     uint32_t launches_per_iteration;
-    uint32_t follow; /* 1: the ant launches take parent-following steps in batches; 2: chosen
-                        every 32 iterations from the walk length */
+    uint32_t follow; /* the ant launches take parent-following steps in batches (by colony, from
+                        its walk length, with FACO_FOLLOW_AUTO): 1 up to one wave of ant warps
+                        or FACO_FOLLOW_ON, 2 beyond one wave */
 } faco_launch_plan;
 int faco_get_launch_plan(faco_engine* engine, faco_launch_plan* plan);
 /* The engine's cudaStream_t (for events recorded by the caller). */
