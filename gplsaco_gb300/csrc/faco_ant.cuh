@@ -211,8 +211,9 @@ __device__ __forceinline__ std::uint32_t pop(const AntSmem& s, Checklist& q, std
 struct AntResult {
     long long construction_cost, final_cost;
     std::uint32_t mne, steps, nonidentity;
-    unsigned long long processed, checks, evaluations, accepted, reactivations;
-    unsigned long long moved;  // tour elements rewritten by relocations and reversals
+    // below 2^32: at most a few pops per accepted move, n moves, 5 w evaluations per pop
+    std::uint32_t processed, checks, evaluations, accepted, reactivations;
+    std::uint32_t moved;  // tour elements rewritten by relocations and reversals, modulo 2^32 (as reported)
     std::uint32_t limit_reached, checklist;
 };
 
@@ -585,11 +586,12 @@ __device__ inline std::uint32_t follow_batch(const AntSmem& s, const int2* xy, c
     return f;
 }
 
-// flip_without_cost (cpp/src/faco_cpu.cpp:114-135) as disjoint swap pairs.
-// Returns the number of elements in the reversed segment.
+// flip_without_cost (cpp/src/faco_cpu.cpp:114-135) between the tour positions
+// of its two end nodes, as disjoint swap pairs.  Returns the number of
+// elements in the reversed segment.  Every lane has read what it needs of the
+// tour before the call's barrier.
 __device__ __forceinline__ std::uint32_t flip(const AntSmem& s, std::uint32_t n, std::uint32_t lane,
-                                              std::uint32_t start, std::uint32_t end) {
-    std::uint32_t first = s.pos[start], last = s.pos[end];
+                                              std::uint32_t first, std::uint32_t last) {
     if (first > last) { const std::uint32_t t = first; first = last; last = t; }
     const std::uint32_t length = last - first;
     const bool straight = length <= n - length || first == 0;
@@ -653,11 +655,13 @@ __device__ __forceinline__ LsRow pop_with_row(const AntSmem& s, Checklist& q, st
 // that fills more than a warp alone (both kinds wide) takes two rounds.
 //
 // Bound by the ant's chain of dependent instructions (one warp issues every
-// ~6 cycles); a pass resolves about two pops for the chain of one.  One GB300,
-// against one pop per pass: one N=100 colony, 64 iterations 8.78 -> 7.46 ms;
-// 256 x 32 ants at N=1000, 320 iterations 151 -> 136 ms; the uneven batch
-// (N 200-1000, 400 iterations) 145 -> 122 ms; 128 x 32 at N=1000-2000, 640
-// iterations 228 -> 205 ms.
+// ~6 cycles; a length takes ~150 cycles, a shuffle 36, a ballot 44); a pass
+// resolves about two pops for the chain of one.  One GB300, against one pop
+// per pass: one N=100 colony, 64 iterations 8.78 -> 7.46 ms; 256 x 32 ants at
+// N=1000, 320 iterations 151 -> 136 ms; the uneven batch (N 200-1000, 400
+// iterations) 145 -> 122 ms; 128 x 32 at N=1000-2000, 640 iterations 228 ->
+// 205 ms.  The winner by one reduction of (node, gain), its payload in two
+// words and the reversal's ends by position: a further 3-6 %.
 constexpr std::uint32_t kPopNodes = 4;
 
 __device__ __forceinline__ void checklist_two_opt(const AntSmem& s, const int2* xy, const InstanceView& in,
@@ -665,7 +669,6 @@ __device__ __forceinline__ void checklist_two_opt(const AntSmem& s, const int2* 
                                                   unsigned long long cap, AntResult& r, long long& gain_sum,
                                                   std::uint32_t* log, std::uint32_t log_cap) {
     const std::uint32_t w = in.w;
-    // evaluations stay far below 2^32 (at most 2 w per pop, a few pops per accepted move, n moves)
     const std::uint32_t limit = cap < 0xffffffffull ? (std::uint32_t)cap : 0xffffffffu;
     std::uint32_t evaluations = 0;
     const std::uint32_t kind = lane & 1u;
@@ -677,11 +680,12 @@ __device__ __forceinline__ void checklist_two_opt(const AntSmem& s, const int2* 
         std::uint32_t at = live ? q.head + i : q.head;
         if (at >= n) at -= n;
         const std::uint32_t a = s.ring[at];
-        std::uint32_t row_b[kPopNodes];
+        std::uint32_t head[kPopNodes], row_b[kPopNodes];
         int row_ab[kPopNodes];
 #pragma unroll
         for (std::uint32_t t = 0; t < kPopNodes; ++t) {
-            const std::size_t row = (std::size_t)__shfl_sync(kFull, a, 2 * t) * w + lane;
+            head[t] = __shfl_sync(kFull, a, 2 * t);
+            const std::size_t row = (std::size_t)head[t] * w + lane;
             row_b[t] = n;
             row_ab[t] = INT_MAX;
             if (lane < w) {
@@ -690,8 +694,10 @@ __device__ __forceinline__ void checklist_two_opt(const AntSmem& s, const int2* 
             }
         }
         const std::uint32_t pa = s.pos[a];
-        const std::uint32_t end = s.tour[kind ? (pa == 0 ? n - 1 : pa - 1) : (pa + 1 == n ? 0 : pa + 1)];
+        const std::uint32_t pend = kind ? (pa == 0 ? n - 1 : pa - 1) : (pa + 1 == n ? 0 : pa + 1);
+        const std::uint32_t end = s.tour[pend];
         const int cur = live ? euc2d(xy[a], xy[end]) : -1;
+        const std::uint32_t ends = a | end << 16;
         // segment ends: off[2i + kind + 1]
         std::uint32_t off[2 * kPopNodes + 1];
         off[0] = 0;
@@ -723,9 +729,11 @@ __device__ __forceinline__ void checklist_two_opt(const AntSmem& s, const int2* 
                 break;
             }
         }
-        // lane t: the t-th candidate of the segments
-        int gain = 0;
-        std::uint32_t best_t = 0, best_seg = 0, best_b = 0, best_nb = 0;
+        // lane t: the t-th candidate of the segments; its best move so far:
+        // the gain, with the first nodes' moves above the others' (lengths
+        // are below 2^25, gains below 2^26)
+        constexpr std::uint32_t kNodeShift = 26;
+        std::uint32_t best = 0, best_ends = 0, best_at = 0;
         for (std::uint32_t base = 0; base < total; base += 32) {
             const std::uint32_t t = base + lane;
             const bool on = t < total;
@@ -737,7 +745,7 @@ __device__ __forceinline__ void checklist_two_opt(const AntSmem& s, const int2* 
             const bool h0 = t >= e0;
             const std::uint32_t seg = on ? (h2 ? 4u : 0u) + (h1 ? 2u : 0u) + (h0 ? 1u : 0u) : 0u;
             const std::uint32_t j = on ? t - (h0 ? e0 : h1 ? e1 : h2 ? off[4] : 0u) : 0u;
-            const std::uint32_t node = __shfl_sync(kFull, a, seg), close = __shfl_sync(kFull, end, seg);
+            const std::uint32_t own = __shfl_sync(kFull, ends, seg), node = own & 0xffffu, close = own >> 16;
             const int edge = __shfl_sync(kFull, cur, seg);
             std::uint32_t b = __shfl_sync(kFull, row_b[0], j);
             int ab = __shfl_sync(kFull, row_ab[0], j);
@@ -749,16 +757,21 @@ __device__ __forceinline__ void checklist_two_opt(const AntSmem& s, const int2* 
             }
             if (on) {
                 const std::uint32_t pb = s.pos[b];
-                const std::uint32_t nb = s.tour[seg & 1u ? (pb == 0 ? n - 1 : pb - 1) : (pb + 1 == n ? 0 : pb + 1)];
+                const std::uint32_t pnb = seg & 1u ? (pb == 0 ? n - 1 : pb - 1) : (pb + 1 == n ? 0 : pb + 1);
+                const std::uint32_t nb = s.tour[pnb];
                 const int2 nxy = xy[nb];
                 const int g = nb == node || b == close ? 0 : edge - ab + euc2d(xy[b], nxy) - euc2d(xy[close], nxy);
-                if (g > gain) { gain = g; best_t = t; best_seg = seg; best_b = b; best_nb = nb; }
+                const std::uint32_t rank = ((kPopNodes - 1 - (seg >> 1)) << kNodeShift) + (std::uint32_t)g;
+                if (g > 0 && rank > best) {
+                    best = rank;
+                    best_ends = b | nb << 16;
+                    best_at = (seg & 1u ? pb : pnb) | seg << 16 | t << 19;   // second end of the reversal, segment, t
+                }
             }
         }
-        const unsigned improving = __ballot_sync(kFull, gain > 0);
         // the pops: up to the first node with a move, else all
-        std::uint32_t popped = nodes;
-        if (improving) popped = (__shfl_sync(kFull, best_seg, __ffs(improving) - 1) >> 1) + 1;
+        const std::uint32_t top = __reduce_max_sync(kFull, best);
+        const std::uint32_t popped = top ? kPopNodes - (top >> kNodeShift) : nodes;
         std::uint32_t done = off[2];
 #pragma unroll
         for (std::uint32_t t = 2; t <= kPopNodes; ++t)
@@ -772,27 +785,33 @@ __device__ __forceinline__ void checklist_two_opt(const AntSmem& s, const int2* 
         q.head += popped;
         if (q.head >= n) q.head -= n;
         q.pending -= popped;
-        for (std::uint32_t t = 0; t < popped; ++t) {   // one at a time: nodes may share a word
-            if (lane == 2 * t) s.queued[a >> 5] &= ~(1u << (a & 31u));
-            __syncwarp();
-        }
-        if (improving) {
-            const bool mine = gain > 0 && (best_seg >> 1) + 1 == popped;
-            const int best = __reduce_max_sync(kFull, mine ? gain : 0);
-            const std::uint32_t first = __reduce_min_sync(kFull, mine && gain == best ? best_t : 0xffu);
-            const std::uint32_t src = first & 31u, seg = __shfl_sync(kFull, best_seg, src);
-            const std::uint32_t bj = __shfl_sync(kFull, best_b, src), nbj = __shfl_sync(kFull, best_nb, src);
-            const std::uint32_t node = __shfl_sync(kFull, a, seg), close = __shfl_sync(kFull, end, seg);
-            // reversed between m0 and m1; all four ends become pending, in this order
+        // pending flags of the pops, each by the lane of its node; lanes that
+        // share a word clear the same bits of it
+        std::uint32_t bits = 0;
+#pragma unroll
+        for (std::uint32_t t = 0; t < kPopNodes; ++t)
+            if (t < popped && (head[t] >> 5) == (a >> 5)) bits |= 1u << (head[t] & 31u);
+        if (lane < 2 * popped && kind == 0) s.queued[a >> 5] &= ~bits;
+        if (top) {
+            // the lowest candidate with that gain, in (kind, rank) order
+            const unsigned ties = __ballot_sync(kFull, best == top);
+            std::uint32_t src = __ffs(ties) - 1;
+            if (total > 32) src = __reduce_min_sync(kFull, best == top ? best_at >> 19 : 0xffu) & 31u;
+            const std::uint32_t move = __shfl_sync(kFull, best_ends, src), at1 = __shfl_sync(kFull, best_at, src);
+            const std::uint32_t seg = (at1 >> 16) & 7u, p1 = at1 & 0xffffu, bj = move & 0xffffu, nbj = move >> 16;
+            const std::uint32_t own = __shfl_sync(kFull, ends, seg), p0 = __shfl_sync(kFull, kind ? pa : pend, seg);
+            const std::uint32_t node = own & 0xffffu, close = own >> 16;
             const bool back = seg & 1u;
+            // all four ends become pending, in this order; reversed between the first two
             const std::uint32_t m0 = back ? node : close, m1 = back ? bj : nbj;
             const std::uint32_t m2 = back ? close : node, m3 = back ? nbj : bj;
-            r.moved += flip(s, n, lane, m0, m1);
+            r.moved += flip(s, n, lane, p0, p1);
             r.reactivations += push_lanes(s, q, n, lane == 0 ? m0 : lane == 1 ? m1 : lane == 2 ? m2 : m3, lane < 4,
                                           lane, log, log_cap);
             ++r.accepted;
-            gain_sum -= best;
+            gain_sum -= (long long)(top & ((1u << kNodeShift) - 1u));
         }
+        __syncwarp();
     }
     r.evaluations += evaluations;
 }
@@ -851,7 +870,7 @@ __device__ __forceinline__ void checklist_ls_first(const AntSmem& s, const int2*
                 std::uint32_t m0, m1, m2, m3;
                 if (kind == 0) { m0 = an; m1 = nbj; m2 = a; m3 = bj; }
                 else { m0 = a; m1 = bj; m2 = ap; m3 = nbj; }
-                r.moved += flip(s, n, lane, m0, m1);
+                r.moved += flip(s, n, lane, s.pos[m0], s.pos[m1]);
                 r.reactivations += push_absent(s, q, n, m0, lane, log, log_cap);
                 r.reactivations += push_absent(s, q, n, m1, lane, log, log_cap);
                 r.reactivations += push_absent(s, q, n, m2, lane, log, log_cap);

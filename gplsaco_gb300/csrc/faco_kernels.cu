@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
         if (lane == 0) s.visited[current >> 5] |= 1u << (current & 31u);
         __syncwarp();
         const float* products = kEngine ? cv.products : L.task_products;
-        const std::uint32_t k = in.k, b = in.b;
+        const std::uint32_t k = in.k;
         const unsigned long long loop_cap = 2ull * n + 2;
         unsigned long long guard = 0;
         // the construction draws of 32 consecutive steps at a time, lane i
@@ -274,12 +274,13 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
                     }
                     selected = __shfl_sync(kFull, cand, j);
                 } else {
+                    const std::uint32_t b = in_ptr->b;   // rare: read where it is used
                     for (std::uint32_t base_j = 0; base_j < b && selected == n; base_j += 32) {
                         const std::uint32_t jj = base_j + lane;
                         std::uint32_t v = n;
                         bool ok = false;
                         if (jj < b) {
-                            v = __ldg(in.backup + (size_t)current * b + jj);
+                            v = __ldg(in_ptr->backup + (size_t)current * b + jj);
                             ok = v < n && !test_bit(s.visited, v);
                         }
                         const unsigned m = __ballot_sync(kFull, ok);
@@ -402,24 +403,28 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
         __syncwarp();
     }
     // ---------------- local search ----------------
+    // (the instance's and the colony's fields are read again where a phase
+    // uses them: kept from the start they would hold 20 registers)
     long long gain_sum = 0;
-    if (L.ls_mode == 1) checklist_ls_first(s, xy, in, n, lane, q, L.ls_limit, r, gain_sum, log, log_cap);
-    else checklist_two_opt(s, xy, in, n, lane, q, L.ls_limit, r, gain_sum, log, log_cap);
+    const InstanceView ls_in = *in_ptr;
+    if (L.ls_mode == 1) checklist_ls_first(s, xy, ls_in, n, lane, q, L.ls_limit, r, gain_sum, log, log_cap);
+    else checklist_two_opt(s, xy, ls_in, n, lane, q, L.ls_limit, r, gain_sum, log, log_cap);
     r.final_cost = cost + gain_sum;
     r.checklist = q.pushed;
     if (log && q.pushed > log_cap && lane == 0) atomicOr(L.error, kErrQueueOverflow);
     __syncwarp();
 
     if (kEngine) {
-        uint4* out = reinterpret_cast<uint4*>(cv.ant_tours + (size_t)ant * cv.n_pad);
+        const ColonyView& to = L.colonies[colony];
+        uint4* out = reinterpret_cast<uint4*>(to.ant_tours + (size_t)ant * to.n_pad);
         const uint4* src = reinterpret_cast<const uint4*>(s.tour);
         for (std::uint32_t c = lane; c * 8 < n; c += 32) out[c] = src[c];
         if (lane == 0) {
-            cv.ant_costs[ant] = r.final_cost;
-            cv.ant_ccosts[ant] = r.construction_cost;
-            cv.ant_counts[3 * ant] = r.steps;
-            cv.ant_counts[3 * ant + 1] = (unsigned)r.evaluations;
-            cv.ant_counts[3 * ant + 2] = (unsigned)r.moved;
+            to.ant_costs[ant] = r.final_cost;
+            to.ant_ccosts[ant] = r.construction_cost;
+            to.ant_counts[3 * ant] = r.steps;
+            to.ant_counts[3 * ant + 1] = (unsigned)r.evaluations;
+            to.ant_counts[3 * ant + 2] = (unsigned)r.moved;
         }
     } else {
         if (L.out_tours)

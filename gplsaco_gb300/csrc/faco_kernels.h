@@ -11,17 +11,18 @@ namespace faco {
 
 // Ants (warps) per block of the ant kernel, and the resident blocks per SM
 // the register budget of each variant is sized for.  Panels that fill the GPU
-// trade registers for resident warps; elsewhere an iteration lasts as long as
-// its slowest ants, and the compiler's longer overlaps (up to 96 and 128
-// registers) pay more than warps that are not there.  One GB300, 4 / 5 / 6 /
-// 7 / 8 blocks: 256 x 32 ants at N=1000, 480 iterations - / 220 / 216 / 216 /
-// 209 ms; the uneven batch (4,096 ant warps) 69.9 / 68.9 / 72.5 / 78.5 / 79.8
-// ms; 32 x 128 ants at N=537 27.1 / 27.7 / 29.3 / 30.1 / 29.9 ms; one N=100
-// colony 4.80 / 4.79 / 5.01 / 5.20 / 5.25 ms; the large panel (global-memory
-// workspace, 2-opt) 497 / 504 / 529 / 542 / 542 ms.
+// trade registers for resident warps (72 registers without room to spare: 8
+// blocks spill); elsewhere an iteration lasts as long as its slowest ants, and
+// the compiler's longer overlaps (up to 96 and 128 registers) pay more than
+// warps that are not there.  One GB300: 256 x 32 ants at N=1000, 320
+// iterations, 7 / 8 blocks: 115.4 / 122.3 ms.  4 / 5 / 6 / 7 / 8 blocks, an
+// earlier build of the same steps: the uneven batch (4,096 ant warps) 69.9 /
+// 68.9 / 72.5 / 78.5 / 79.8 ms; 32 x 128 ants at N=537 27.1 / 27.7 / 29.3 /
+// 30.1 / 29.9 ms; one N=100 colony 4.80 / 4.79 / 5.01 / 5.20 / 5.25 ms; the
+// large panel (global-memory workspace, 2-opt) 497 / 504 / 529 / 542 / 542 ms.
 constexpr std::uint32_t kMaxWarpsPerBlock = 4;
 constexpr std::uint32_t ant_blocks_per_sm(int mode) {
-    return dense_mode(mode) ? 8 : global_mode(mode) ? 4 : follow_mode(mode) ? 5 : 6;
+    return dense_mode(mode) ? 7 : global_mode(mode) ? 4 : follow_mode(mode) ? 5 : 6;
 }
 
 struct ColonyParams {
