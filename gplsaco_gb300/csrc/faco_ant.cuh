@@ -47,16 +47,24 @@ enum AntMode : int {
     kModeEngineFollowDense = 7,
 };
 
+// An engine variant compiled for one local search (or'ed to the mode).  With
+// both in one kernel the register budget of the larger one spills in the
+// other: 256 x 32 ants at N=1000 ran 122.5 ms instead of 115.4.
+constexpr int kTwoOptOnly = 16, kOrOptOnly = 32, kModeMask = 15;
+
 __host__ __device__ constexpr bool engine_mode(int mode) {
-    return mode == kModeEngine || mode == kModeEngineGlobal || mode == kModeEngineFollow ||
-           mode == kModeEngineGlobalFollow || mode == kModeEngineFollowDense;
+    const int m = mode & kModeMask;
+    return m == kModeEngine || m == kModeEngineGlobal || m == kModeEngineFollow || m == kModeEngineGlobalFollow ||
+           m == kModeEngineFollowDense;
 }
 __host__ __device__ constexpr bool global_mode(int mode) {
-    return mode == kModeEngineGlobal || mode == kModeEngineGlobalFollow;
+    const int m = mode & kModeMask;
+    return m == kModeEngineGlobal || m == kModeEngineGlobalFollow;
 }
-__host__ __device__ constexpr bool dense_mode(int mode) { return mode == kModeEngineFollowDense; }
+__host__ __device__ constexpr bool dense_mode(int mode) { return (mode & kModeMask) == kModeEngineFollowDense; }
 __host__ __device__ constexpr bool follow_mode(int mode) {
-    return mode == kModeEngineFollow || mode == kModeEngineGlobalFollow || mode == kModeEngineFollowDense;
+    const int m = mode & kModeMask;
+    return m == kModeEngineFollow || m == kModeEngineGlobalFollow || m == kModeEngineFollowDense;
 }
 // The batched variant of an engine mode (`dense`: the build for panels
 // beyond one wave, where there is one).
@@ -152,26 +160,6 @@ struct Checklist {
     std::uint32_t head, tail, pending, pushed;  // ring indices and counters (warp-uniform)
 };
 
-// Appends v unless it is pending (reference append_if_absent,
-// cuda/faco_device.cuh:81-92).  Warp-uniform decision, lane 0 stores.
-__device__ __forceinline__ bool push_absent(const AntSmem& s, Checklist& q, std::uint32_t n, std::uint32_t v,
-                                            std::uint32_t lane, std::uint32_t* log, std::uint32_t log_cap) {
-    const bool absent = !test_bit(s.queued, v);
-    __syncwarp();   // every lane has read the flag before lane 0 sets it
-    if (absent) {
-        if (lane == 0) {
-            s.queued[v >> 5] |= 1u << (v & 31u);
-            s.ring[q.tail] = (node_t)v;
-            if (log && q.pushed < log_cap) log[q.pushed] = v;
-        }
-        q.tail = q.tail + 1 == n ? 0 : q.tail + 1;
-        ++q.pending;
-        ++q.pushed;
-    }
-    __syncwarp();
-    return absent;
-}
-
 // Appends the nodes of lanes 0, 1, ... (each lane its own `v`, taken when
 // `want`) that are not pending, in lane order: what one append_if_absent
 // after the other does (cuda/faco_device.cuh:81-92).  The wanted nodes are
@@ -196,16 +184,6 @@ __device__ __forceinline__ std::uint32_t push_lanes(const AntSmem& s, Checklist&
     q.pushed += count;
     __syncwarp();
     return count;
-}
-
-__device__ __forceinline__ std::uint32_t pop(const AntSmem& s, Checklist& q, std::uint32_t n,
-                                             std::uint32_t lane) {
-    const std::uint32_t a = s.ring[q.head];
-    q.head = q.head + 1 == n ? 0 : q.head + 1;
-    --q.pending;
-    __syncwarp();
-    if (lane == 0) s.queued[a >> 5] &= ~(1u << (a & 31u));
-    return a;
 }
 
 struct AntResult {
@@ -609,33 +587,6 @@ __device__ __forceinline__ std::uint32_t flip(const AntSmem& s, std::uint32_t n,
     return count;
 }
 
-// LS row of one node: candidate id and its cached distance, one per lane.
-struct LsRow {
-    std::uint32_t node, b;
-    int ab;
-};
-__device__ __forceinline__ LsRow load_row(const InstanceView& in, std::uint32_t a, std::uint32_t lane) {
-    LsRow r{a, in.n, 0};
-    if (lane < in.w) {
-        r.b = __ldg(in.ls + (size_t)a * in.w + lane);
-        r.ab = __ldg(in.ls_dist + (size_t)a * in.w + lane);
-    }
-    return r;
-}
-
-// Pops the next pending node and returns its LS row, taking the prefetched
-// row when it belongs to that node; then prefetches the row of the node now
-// at the head (it cannot change before it is popped).
-__device__ __forceinline__ LsRow pop_with_row(const AntSmem& s, Checklist& q, std::uint32_t n,
-                                              std::uint32_t lane, const InstanceView& in, LsRow& next) {
-    const std::uint32_t a = pop(s, q, n, lane);
-    LsRow row = next.node == a ? next : load_row(in, a, lane);
-    row.node = a;
-    next.node = n;
-    if (q.pending > 0) next = load_row(in, s.ring[q.head], lane);
-    return row;
-}
-
 // Checklist 2-opt, best gain per popped node, reference tie/cap rules
 // (cpp/src/faco_cpu.cpp:148-217; cuda/faco_device.cuh:295-478).
 //
@@ -819,140 +770,275 @@ __device__ __forceinline__ void checklist_two_opt(const AntSmem& s, const int2* 
 // Checklist local search with first-improvement 2-opt then Or-opt (segments
 // of 1-3 nodes starting at the popped node).  The reference has no Or-opt;
 // the move order, pruning and counting rules are this engine's own (stated in
-// full beside the CPU restatement).  Every lane evaluates one candidate; the
-// first improving move in scan order is found with one ballot.
+// full beside the CPU restatement).
+//
+// As in checklist_two_opt, up to kPopNodes pops are evaluated together and
+// those up to the first with a move are taken: lanes 8i + r hold node i's
+// tour neighbourhood (the nodes at positions -1 .. +3 around it, r = 0 .. 4)
+// and its five scans (r = 0, 1: the 2-opt kinds; 2-4: the Or-opt lengths).
+// Every move is the same expression: a candidate c of the node's row joins
+// its tour neighbour nb on one side of it,
+//   gain = base + d(c, nb) - d(a, c) - d(X, nb),
+// base and X belonging to the scan.  The 2-opt scans of all nodes go one
+// candidate per lane; then, node by node up to the first one with a 2-opt
+// move, its Or-opt scans, one (candidate, side) per lane in scan order, so
+// that the lowest lane with a gain is the first improvement.  On instances
+// in the global-memory workspace a pop is a chain of five L2 reads, which the
+// nodes of a pass share.  One GB300, the large panel (80 colonies x 64 ants,
+// N 5000-10000, 80 iterations): 132 -> 110 ms.
 __device__ __forceinline__ void checklist_ls_first(const AntSmem& s, const int2* xy, const InstanceView& in,
                                                    std::uint32_t n, std::uint32_t lane, Checklist& q,
                                                    unsigned long long cap, AntResult& r, long long& gain_sum,
                                                    std::uint32_t* log, std::uint32_t log_cap) {
     const std::uint32_t w = in.w;
-    LsRow next{n, n, 0};
+    const std::uint32_t limit = cap < 0xffffffffull ? (std::uint32_t)cap : 0xffffffffu;
+    const std::uint32_t lengths = n < 6 ? n - 3 : 3u;   // Or-opt lengths L with n >= L + 3
+    std::uint32_t evaluations = 0;
+    const std::uint32_t role = lane & 7u, first = lane & 24u;
+    // scan tests of a row whose first f candidates pass
+    const auto scanned = [&](std::uint32_t f) { return f + (f < w ? 1u : 0u); };
     while (q.pending > 0 && r.accepted < n) {
-        if (r.evaluations >= cap) { r.limit_reached = 1; break; }
-        const LsRow row = pop_with_row(s, q, n, lane, in, next);
-        const std::uint32_t a = row.node, c = row.b;
-        const int ac = row.ab;
-        const std::uint32_t pa = s.pos[a];
-        const std::uint32_t an = s.tour[pa + 1 == n ? 0 : pa + 1];
-        const std::uint32_t ap = s.tour[pa == 0 ? n - 1 : pa - 1];
-        ++r.processed;
-        const int2 a_xy = xy[a];
-        const int cur0 = euc2d(a_xy, xy[an]), cur1 = euc2d(xy[ap], a_xy);
-        const bool valid = lane < w && c < n;
-        std::uint32_t pc = 0, c_next = 0, c_prev = 0;
-        int2 c_xy = make_int2(0, 0);
-        if (valid) {
-            pc = s.pos[c];
-            c_next = s.tour[pc + 1 == n ? 0 : pc + 1];
-            c_prev = s.tour[pc == 0 ? n - 1 : pc - 1];
-            c_xy = xy[c];
+        if (evaluations >= limit) { r.limit_reached = 1; break; }
+        const bool live = (lane >> 3) < q.pending;
+        std::uint32_t at = live ? q.head + (lane >> 3) : q.head;
+        if (at >= n) at -= n;
+        const std::uint32_t a = s.ring[at];
+        std::uint32_t head[kPopNodes], row_b[kPopNodes];
+        int row_ab[kPopNodes];
+#pragma unroll
+        for (std::uint32_t t = 0; t < kPopNodes; ++t) {
+            head[t] = __shfl_sync(kFull, a, 8 * t);
+            const std::size_t row = (std::size_t)head[t] * w + lane;
+            row_b[t] = n;
+            row_ab[t] = INT_MAX;
+            if (lane < w) {
+                row_b[t] = __ldg(in.ls + row);
+                row_ab[t] = __ldg(in.ls_dist + row);
+            }
+            if (row_b[t] >= n) row_ab[t] = INT_MAX;   // right padding
         }
-        bool interrupted = false, found = false;
-        // ---- 2-opt, first improvement in (kind, j) order
-        for (std::uint32_t kind = 0; kind < 2 && !found && !interrupted; ++kind) {
-            const int cur = kind == 0 ? cur0 : cur1;
-            const std::uint32_t closing_end = kind == 0 ? an : ap;
-            const unsigned badm = __ballot_sync(kFull, lane < w && (!valid || !(cur > ac)));
-            const std::uint32_t f = badm ? __ffs(badm) - 1 : w;
-            const unsigned long long remaining = cap - r.evaluations;
-            const std::uint32_t used = remaining < f ? (std::uint32_t)remaining : f;
-            int g = INT_MIN;
-            const std::uint32_t nb = kind == 0 ? c_next : c_prev;
-            if (lane < used)
-                g = (nb == a || c == closing_end) ? 0 : cur + euc2d(c_xy, xy[nb]) - ac - euc2d(xy[closing_end], xy[nb]);
-            const unsigned improving = __ballot_sync(kFull, lane < used && g > 0);
+        // tour nodes t0 .. t4 at positions -1 .. +3, roles 0 .. 4
+        std::uint32_t at_tour = s.pos[a] + n - 1 + (role < 5 ? role : 1u);
+        if (at_tour >= n) at_tour -= n;
+        if (at_tour >= n) at_tour -= n;
+        const std::uint32_t near = s.tour[at_tour];
+        const int2 near_xy = xy[near];
+        // roles 0-3: d(t_r, t_r+1); roles 4-6: d(t0, t_r-2)
+        const std::uint32_t from = first + (role < 4 ? role : 0u), to = first + (role < 4 ? role + 1 : role < 7 ? role - 2 : 0u);
+        const int2 p = make_int2(__shfl_sync(kFull, near_xy.x, from), __shfl_sync(kFull, near_xy.y, from));
+        const int2 o = make_int2(__shfl_sync(kFull, near_xy.x, to), __shfl_sync(kFull, near_xy.y, to));
+        const int d = euc2d(p, o);
+        // scan bases: d(a, next), d(prev, a), and the removal gains
+        // d(prev, a) + d(e, q) - d(prev, q) of the segments a .. e before q
+        const int d0 = __shfl_sync(kFull, d, role == 0 ? first + 1 : first);
+        const int deq = __shfl_sync(kFull, d, first + (role >= 2 ? role - 1 : 0u));
+        const int dpq = __shfl_sync(kFull, d, first + (role >= 2 && role < 5 ? role + 2 : 0u));
+        const std::uint32_t X = __shfl_sync(kFull, near, first + (role == 0 ? 2u : role == 1 ? 0u : role < 5 ? role - 1 : 0u));
+        const int base = !live || role > 1 + lengths ? -1 : role < 2 ? d0 : d0 + deq - dpq;
+        // the 2-opt scans, as in checklist_two_opt
+        std::uint32_t off[2 * kPopNodes + 1];
+        off[0] = 0;
+#pragma unroll
+        for (std::uint32_t g = 0; g < 2 * kPopNodes; ++g) {
+            const int c = __shfl_sync(kFull, base, 8 * (g >> 1) + (g & 1u));
+            off[g + 1] = off[g] + __popc(__ballot_sync(kFull, c > row_ab[g >> 1]));
+        }
+        std::uint32_t nodes = 1;
+#pragma unroll
+        for (std::uint32_t t = 2; t <= kPopNodes; ++t)
+            if (off[2 * t] <= 32u) nodes = t;
+        nodes = nodes < q.pending ? nodes : q.pending;
+        // near the end of the budget one node at a time, cut where it ends
+        const std::uint32_t left = limit - evaluations;
+        const bool tight = left <= 5 * kPopNodes * 32;
+        if (tight) nodes = 1;
+        std::uint32_t total = off[2];
+#pragma unroll
+        for (std::uint32_t t = 2; t <= kPopNodes; ++t)
+            if (nodes == t) total = off[2 * t];
+        bool two_opt = false;
+        std::uint32_t move_c = 0, move_nb = 0, move_seg = 0, move_t = 0, node_of = nodes;
+        int move_gain = 0;
+        for (std::uint32_t base_t = 0; base_t < total && !two_opt; base_t += 32) {
+            const std::uint32_t t = base_t + lane;
+            const bool on = t < total;
+            const bool h2 = t >= off[4];
+            const std::uint32_t e1 = h2 ? off[6] : off[2];
+            const bool h1 = t >= e1;
+            const std::uint32_t e0 = h2 ? (h1 ? off[7] : off[5]) : (h1 ? off[3] : off[1]);
+            const bool h0 = t >= e0;
+            const std::uint32_t seg = on ? (h2 ? 4u : 0u) + (h1 ? 2u : 0u) + (h0 ? 1u : 0u) : 0u;
+            const std::uint32_t j = on ? t - (h0 ? e0 : h1 ? e1 : h2 ? off[4] : 0u) : 0u;
+            const std::uint32_t own = 8 * (seg >> 1) + (seg & 1u);
+            const std::uint32_t close = __shfl_sync(kFull, X, own), node = __shfl_sync(kFull, a, own);
+            const int edge = __shfl_sync(kFull, base, own);
+            std::uint32_t c = __shfl_sync(kFull, row_b[0], j);
+            int ac = __shfl_sync(kFull, row_ab[0], j);
+#pragma unroll
+            for (std::uint32_t x = 1; x < kPopNodes; ++x) {
+                const std::uint32_t cx = __shfl_sync(kFull, row_b[x], j);
+                const int acx = __shfl_sync(kFull, row_ab[x], j);
+                if ((seg >> 1) == x) { c = cx; ac = acx; }
+            }
+            int g = 0;
+            std::uint32_t nb = 0;
+            if (on) {
+                const std::uint32_t pc = s.pos[c];
+                nb = s.tour[seg & 1u ? (pc == 0 ? n - 1 : pc - 1) : (pc + 1 == n ? 0 : pc + 1)];
+                const int2 nxy = xy[nb];
+                g = nb == node || c == close ? 0 : edge - ac + euc2d(xy[c], nxy) - euc2d(xy[close], nxy);
+            }
+            const unsigned improving = __ballot_sync(kFull, g > 0);
             if (improving) {
-                const std::uint32_t j = __ffs(improving) - 1;
-                r.evaluations += j + 1;
-                r.checks += j + 1;
-                const int gain = __shfl_sync(kFull, g, j);
-                const std::uint32_t bj = __shfl_sync(kFull, c, j), nbj = __shfl_sync(kFull, nb, j);
-                std::uint32_t m0, m1, m2, m3;
-                if (kind == 0) { m0 = an; m1 = nbj; m2 = a; m3 = bj; }
-                else { m0 = a; m1 = bj; m2 = ap; m3 = nbj; }
-                r.moved += flip(s, n, lane, s.pos[m0], s.pos[m1]);
-                r.reactivations += push_absent(s, q, n, m0, lane, log, log_cap);
-                r.reactivations += push_absent(s, q, n, m1, lane, log, log_cap);
-                r.reactivations += push_absent(s, q, n, m2, lane, log, log_cap);
-                r.reactivations += push_absent(s, q, n, m3, lane, log, log_cap);
-                ++r.accepted;
-                gain_sum -= gain;
-                found = true;
-            } else {
-                r.evaluations += used;
-                r.checks += used + (used < w ? 1 : 0);
-                if (used < f) interrupted = true;
+                const std::uint32_t src = __ffs(improving) - 1;
+                two_opt = true;
+                move_c = __shfl_sync(kFull, c, src);
+                move_nb = __shfl_sync(kFull, nb, src);
+                move_seg = __shfl_sync(kFull, seg, src);
+                move_t = base_t + src;
+                node_of = move_seg >> 1;
+                move_gain = __shfl_sync(kFull, g, src);
             }
         }
-        if (interrupted) { r.limit_reached = 1; break; }
-        if (found) {
-            __syncwarp();
-            continue;
-        }
-        // ---- Or-opt: segment a.. of L nodes, first improvement in (L, j, variant) order
-        std::uint32_t seg0 = a, seg1 = n, seg2 = n;
-        const int d_pa = cur1;
-        for (std::uint32_t L = 1; L <= 3 && !found && !interrupted; ++L) {
-            if (n < L + 3) break;
-            if (L == 2) seg1 = an;
-            if (L == 3) { const std::uint32_t p1 = s.pos[seg1]; seg2 = s.tour[p1 + 1 == n ? 0 : p1 + 1]; }
-            const std::uint32_t e = L == 1 ? seg0 : L == 2 ? seg1 : seg2;
-            const std::uint32_t pe = s.pos[e];
-            const std::uint32_t qn = s.tour[pe + 1 == n ? 0 : pe + 1];
-            const int2 e_xy = xy[e];
-            const int G = d_pa + euc2d(e_xy, xy[qn]) - euc2d(xy[ap], xy[qn]);
-            const unsigned badm = __ballot_sync(kFull, lane < w && (!valid || !(G > ac)));
-            const std::uint32_t f = badm ? __ffs(badm) - 1 : w;
-            const unsigned long long remaining = cap - r.evaluations;
-            const std::uint32_t used = remaining < f ? (std::uint32_t)remaining : f;
-            int g1 = INT_MIN, g2 = INT_MIN;
-            if (lane < used) {
-                const bool inside = c == seg0 || c == seg1 || c == seg2;
-                if (!inside) {
-                    if (!(c_next == seg0 || c_next == seg1 || c_next == seg2))
-                        g1 = G + euc2d(c_xy, xy[c_next]) - ac - euc2d(e_xy, xy[c_next]);
-                    if (!(c_prev == seg0 || c_prev == seg1 || c_prev == seg2))
-                        g2 = G + euc2d(xy[c_prev], c_xy) - euc2d(xy[c_prev], e_xy) - ac;
+        // the Or-opt scans of the nodes before it (of all, without one)
+        bool or_opt = false;
+        std::uint32_t or_c = 0, or_nb = 0, or_len = 0, or_side = 0, or_done = 0, or_node = 0;
+        std::uint32_t f1 = 0, f2 = 0, f3 = 0, checks = 0;
+        int or_gain = 0;
+        for (std::uint32_t i = 0; i < node_of && !or_opt; ++i) {
+            std::uint32_t rb = row_b[0], ai = head[0];
+            int rab = row_ab[0];
+#pragma unroll
+            for (std::uint32_t x = 1; x < kPopNodes; ++x)
+                if (i == x) { rb = row_b[x]; rab = row_ab[x]; ai = head[x]; }
+            const std::uint32_t own = 8 * i + 2;
+            const int g1 = __shfl_sync(kFull, base, own), g2 = __shfl_sync(kFull, base, own + 1);
+            const int g3 = __shfl_sync(kFull, base, own + 2);
+            const std::uint32_t s2 = __shfl_sync(kFull, near, own), s3 = __shfl_sync(kFull, near, own + 1);
+            f1 = __popc(__ballot_sync(kFull, g1 > rab));
+            f2 = __popc(__ballot_sync(kFull, g2 > rab));
+            f3 = __popc(__ballot_sync(kFull, g3 > rab));
+            const std::uint32_t o1 = 2 * f1, o2 = o1 + 2 * f2, o3 = o2 + 2 * f3;
+            for (std::uint32_t base_t = 0; base_t < o3 && !or_opt; base_t += 32) {
+                const std::uint32_t t = base_t + lane;
+                const bool on = t < o3;
+                const std::uint32_t len = on ? (t >= o1 ? 1u : 0u) + (t >= o2 ? 1u : 0u) : 0u;   // L - 1
+                const std::uint32_t rest = on ? t - (len == 0 ? 0u : len == 1 ? o1 : o2) : 0u;
+                const std::uint32_t j = rest >> 1, side = rest & 1u;   // side 0: between c and its successor
+                const std::uint32_t c = __shfl_sync(kFull, rb, j), e = __shfl_sync(kFull, X, own + len);
+                const int ac = __shfl_sync(kFull, rab, j), G = __shfl_sync(kFull, base, own + len);
+                const auto inside = [&](std::uint32_t v) {
+                    return v == ai || (len >= 1 && v == s2) || (len >= 2 && v == s3);
+                };
+                int g = 0;
+                std::uint32_t nb = 0;
+                if (on) {
+                    const std::uint32_t pc = s.pos[c];
+                    nb = s.tour[side ? (pc == 0 ? n - 1 : pc - 1) : (pc + 1 == n ? 0 : pc + 1)];
+                    const int2 nxy = xy[nb];
+                    g = inside(c) || inside(nb) ? 0 : G - ac + euc2d(xy[c], nxy) - euc2d(xy[e], nxy);
+                }
+                const unsigned improving = __ballot_sync(kFull, g > 0);
+                if (improving) {
+                    const std::uint32_t src = __ffs(improving) - 1;
+                    or_opt = true;
+                    or_node = i;
+                    or_c = __shfl_sync(kFull, c, src);
+                    or_nb = __shfl_sync(kFull, nb, src);
+                    or_len = __shfl_sync(kFull, len, src) + 1;
+                    or_side = __shfl_sync(kFull, side, src);
+                    or_gain = __shfl_sync(kFull, g, src);
+                    f3 = or_len >= 3 ? __shfl_sync(kFull, j, src) + 1 : 0u;
+                    f2 = or_len == 2 ? __shfl_sync(kFull, j, src) + 1 : or_len > 2 ? f2 : 0u;
+                    f1 = or_len == 1 ? __shfl_sync(kFull, j, src) + 1 : f1;
                 }
             }
-            const unsigned improving = __ballot_sync(kFull, lane < used && (g1 > 0 || g2 > 0));
-            if (improving) {
-                const std::uint32_t j = __ffs(improving) - 1;
-                r.evaluations += j + 1;
-                r.checks += j + 1;
-                const int g1j = __shfl_sync(kFull, g1, j), g2j = __shfl_sync(kFull, g2, j);
-                const std::uint32_t cj = __shfl_sync(kFull, c, j);
-                const std::uint32_t c2 = __shfl_sync(kFull, c_next, j), c0 = __shfl_sync(kFull, c_prev, j);
-                const bool first_variant = g1j > 0;
-                // (i) c, a .. e, c2: relocate a after c, then each next node after the last moved
-                // (ii) c0, e .. a, c: relocate e after c0, then each previous node
-                std::uint32_t target = first_variant ? cj : c0;
-                for (std::uint32_t t = 0; t < L; ++t) {
-                    const std::uint32_t idx = first_variant ? t : L - 1 - t;
-                    const std::uint32_t node = idx == 0 ? seg0 : idx == 1 ? seg1 : seg2;
-                    const std::uint32_t tp = s.pos[target], np = s.pos[node];
-                    relocate_shift(s, lane, tp, np, node);
-                    r.moved += tp < np ? np - tp : tp - np + 1;
-                    target = node;
-                }
-                r.reactivations += push_absent(s, q, n, ap, lane, log, log_cap);
-                r.reactivations += push_absent(s, q, n, a, lane, log, log_cap);
-                r.reactivations += push_absent(s, q, n, e, lane, log, log_cap);
-                r.reactivations += push_absent(s, q, n, qn, lane, log, log_cap);
-                r.reactivations += push_absent(s, q, n, first_variant ? cj : c0, lane, log, log_cap);
-                r.reactivations += push_absent(s, q, n, first_variant ? c2 : cj, lane, log, log_cap);
-                ++r.accepted;
-                gain_sum -= first_variant ? g1j : g2j;
-                found = true;
-            } else {
-                r.evaluations += used;
-                r.checks += used + (used < w ? 1 : 0);
-                if (used < f) interrupted = true;
-            }
+            or_done += f1 + f2 + f3;
+            // scan tests: whole scans, the last one up to its move
+            const std::uint32_t whole = or_opt ? or_len - 1 : lengths;
+            checks += (whole >= 1 ? scanned(f1) : f1) + (whole >= 2 ? scanned(f2) : f2) +
+                      (whole >= 3 ? scanned(f3) : f3);
         }
-        if (interrupted) { r.limit_reached = 1; break; }
+        // (an Or-opt move, of an earlier node, comes before the 2-opt one)
+        const std::uint32_t popped = or_opt ? or_node + 1 : two_opt ? node_of + 1 : nodes;
+        std::uint32_t before = 0;   // 2-opt evaluations of the pops, or up to the 2-opt move
+#pragma unroll
+        for (std::uint32_t t = 1; t <= kPopNodes; ++t)
+            if (popped == t) before = off[2 * t];
+        if (two_opt && !or_opt) before = move_t + 1;
+        if (tight && before + or_done > left) {
+            // the budget ends inside this node's scans
+            std::uint32_t rest = left;
+            const std::uint32_t f[5] = {off[1], off[2] - off[1], f1, f2, f3};
+#pragma unroll
+            for (std::uint32_t g = 0; g < 5; ++g) {
+                if (g >= 2 + lengths || rest == 0xffffffffu) continue;
+                const std::uint32_t used = rest < f[g] ? rest : f[g];
+                r.checks += scanned(used);
+                rest = used < f[g] ? 0xffffffffu : rest - used;
+            }
+            evaluations += left;
+            ++r.processed;
+            r.limit_reached = 1;
+            break;
+        }
+        evaluations += before + or_done;
+        r.processed += popped;
+        r.checks += checks;
+#pragma unroll
+        for (std::uint32_t g = 0; g < 2 * kPopNodes; ++g) {
+            if ((g >> 1) >= popped) continue;
+            const std::uint32_t f = off[g + 1] - off[g];
+            if (or_opt || !two_opt || g < move_seg) r.checks += scanned(f);
+            else if (g == move_seg) r.checks += move_t + 1 - off[g];
+        }
+        q.head += popped;
+        if (q.head >= n) q.head -= n;
+        q.pending -= popped;
+        // pending flags of the pops; lanes that share a word clear the same bits of it
+        std::uint32_t bits = 0;
+#pragma unroll
+        for (std::uint32_t t = 0; t < kPopNodes; ++t)
+            if (t < popped && (head[t] >> 5) == (a >> 5)) bits |= 1u << (head[t] & 31u);
+        if (role == 0 && (lane >> 3) < popped) s.queued[a >> 5] &= ~bits;
         __syncwarp();
+        if (or_opt) {
+            const std::uint32_t own = 8 * or_node;
+            const std::uint32_t prev = __shfl_sync(kFull, near, own), node = __shfl_sync(kFull, near, own + 1);
+            const std::uint32_t e = __shfl_sync(kFull, near, own + or_len), next = __shfl_sync(kFull, near, own + or_len + 1);
+            // (0) c, a .. e, c2: a goes after c, then each next node after the last moved
+            // (1) c0, e .. a, c: e goes after c0, then each previous node
+            std::uint32_t target = or_side ? or_nb : or_c;
+            for (std::uint32_t t = 0; t < or_len; ++t) {
+                const std::uint32_t moved = __shfl_sync(kFull, near, own + 1 + (or_side ? or_len - 1 - t : t));
+                const std::uint32_t tp = s.pos[target], np = s.pos[moved];
+                relocate_shift(s, lane, tp, np, moved);
+                r.moved += tp < np ? np - tp : tp - np + 1;
+                target = moved;
+            }
+            const std::uint32_t v = lane == 0 ? prev : lane == 1 ? node : lane == 2 ? e : lane == 3 ? next
+                                  : lane == 4 ? (or_side ? or_nb : or_c) : (or_side ? or_c : or_nb);
+            bool want = lane < 6;
+#pragma unroll
+            for (std::uint32_t t = 0; t < 5; ++t)
+                if (__shfl_sync(kFull, v, t) == v && t < lane) want = false;   // already in the list
+            r.reactivations += push_lanes(s, q, n, v, want, lane, log, log_cap);
+            ++r.accepted;
+            gain_sum -= or_gain;
+        } else if (two_opt) {
+            const std::uint32_t own = 8 * node_of + (move_seg & 1u);
+            const std::uint32_t node = __shfl_sync(kFull, a, own), close = __shfl_sync(kFull, X, own);
+            const bool back = move_seg & 1u;
+            const std::uint32_t m0 = back ? node : close, m1 = back ? move_c : move_nb;
+            const std::uint32_t m2 = back ? close : node, m3 = back ? move_nb : move_c;
+            r.moved += flip(s, n, lane, s.pos[m0], s.pos[m1]);
+            r.reactivations += push_lanes(s, q, n, lane == 0 ? m0 : lane == 1 ? m1 : lane == 2 ? m2 : m3, lane < 4,
+                                          lane, log, log_cap);
+            ++r.accepted;
+            gain_sum -= move_gain;
+        }
     }
+    r.evaluations += evaluations;
 }
 
 }  // namespace faco

@@ -251,7 +251,7 @@ std::vector<std::uint32_t> parent_neighbours(const std::uint32_t* tour, std::uin
 
 void launch_ants(int mode, const faco::AntLaunch& L, std::uint32_t blocks, std::uint32_t warps, cudaStream_t s) {
     const std::uint32_t smem = faco::block_smem_bytes(L.n_max, warps);
-    cuda_check(faco::prepare_ant_kernel(mode, smem), "cudaFuncSetAttribute");
+    cuda_check(faco::prepare_ant_kernel(mode, L.ls_mode, smem), "cudaFuncSetAttribute");
     cuda_check(faco::launch_ant_kernel(mode, L, blocks, warps, smem, s), "ant kernel launch");
 }
 
@@ -808,7 +808,7 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
                     const auto jobs = jobs_for(members[i], w);
                     e->work.upload(jobs, s);
                     const faco::AntLaunch L = launch_of(0, w, cl.n_max);
-                    cuda_check(faco::prepare_ant_kernel(timed, smem), "attribute");
+                    cuda_check(faco::prepare_ant_kernel(timed, c.ls_mode, smem), "attribute");
                     float ms = 0.0f;
                     for (int rep = 0; rep < 3; ++rep) {
                         cuda_check(cudaEventRecord(t0, s), "event");
@@ -887,7 +887,7 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
     }
     for (auto& ch : v.chains) ch.L = launch_of(ch.first_job, v.classes[ch.cls].warps, v.classes[ch.cls].n_max);
     for (const auto& [mode, smem] : smem_max)
-        if (smem) cuda_check(faco::prepare_ant_kernel(mode, smem), "cudaFuncSetAttribute");
+        if (smem) cuda_check(faco::prepare_ant_kernel(mode, c.ls_mode, smem), "cudaFuncSetAttribute");
 }
 
 // Controller programs of a GP-controlled evaluation (null: plain FACO).

@@ -13,6 +13,7 @@
 //                           (cuda/gp_score.cuh:64-102)
 #include <mutex>
 #include <climits>
+#include <type_traits>
 
 #include "faco_ant.cuh"
 #include "faco_kernels.h"
@@ -407,7 +408,7 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
     // uses them: kept from the start they would hold 20 registers)
     long long gain_sum = 0;
     const InstanceView ls_in = *in_ptr;
-    if (L.ls_mode == 1) checklist_ls_first(s, xy, ls_in, n, lane, q, L.ls_limit, r, gain_sum, log, log_cap);
+    if ((MODE & kOrOptOnly) || (!(MODE & kTwoOptOnly) && L.ls_mode == 1)) checklist_ls_first(s, xy, ls_in, n, lane, q, L.ls_limit, r, gain_sum, log, log_cap);
     else checklist_two_opt(s, xy, ls_in, n, lane, q, L.ls_limit, r, gain_sum, log, log_cap);
     r.final_cost = cost + gain_sum;
     r.checklist = q.pushed;
@@ -467,35 +468,39 @@ cudaError_t prepare_mode(std::uint32_t smem) {
 }
 }  // namespace
 
-cudaError_t prepare_ant_kernel(int mode, std::uint32_t smem) {
+namespace {
+// f(variant) for the kernel variant of a mode and local search.
+template <class F>
+cudaError_t for_variant(int mode, std::uint32_t ls_mode, F&& f) {
+    const auto engine = [&](auto m) {
+        constexpr int kMode = decltype(m)::value;
+        return ls_mode == 1 ? f(std::integral_constant<int, kMode | kOrOptOnly>{})
+                            : f(std::integral_constant<int, kMode | kTwoOptOnly>{});
+    };
     switch (mode) {
-        case kModeEngine: return prepare_mode<kModeEngine>(smem);
-        case kModeVisits: return prepare_mode<kModeVisits>(smem);
-        case kModeUniforms: return prepare_mode<kModeUniforms>(smem);
-        case kModePrepare: return prepare_mode<kModePrepare>(smem);
-        case kModeEngineGlobal: return prepare_mode<kModeEngineGlobal>(smem);
-        case kModeEngineFollow: return prepare_mode<kModeEngineFollow>(smem);
-        case kModeEngineGlobalFollow: return prepare_mode<kModeEngineGlobalFollow>(smem);
-        case kModeEngineFollowDense: return prepare_mode<kModeEngineFollowDense>(smem);
+        case kModeEngine: return engine(std::integral_constant<int, kModeEngine>{});
+        case kModeVisits: return f(std::integral_constant<int, kModeVisits>{});
+        case kModeUniforms: return f(std::integral_constant<int, kModeUniforms>{});
+        case kModePrepare: return f(std::integral_constant<int, kModePrepare>{});
+        case kModeEngineGlobal: return engine(std::integral_constant<int, kModeEngineGlobal>{});
+        case kModeEngineFollow: return engine(std::integral_constant<int, kModeEngineFollow>{});
+        case kModeEngineGlobalFollow: return engine(std::integral_constant<int, kModeEngineGlobalFollow>{});
+        case kModeEngineFollowDense: return engine(std::integral_constant<int, kModeEngineFollowDense>{});
         default: return cudaErrorInvalidValue;
     }
+}
+}  // namespace
+
+cudaError_t prepare_ant_kernel(int mode, std::uint32_t ls_mode, std::uint32_t smem) {
+    return for_variant(mode, ls_mode, [&](auto m) { return prepare_mode<decltype(m)::value>(smem); });
 }
 
 cudaError_t launch_ant_kernel(int mode, const AntLaunch& L, std::uint32_t blocks, std::uint32_t warps,
                               std::uint32_t smem, cudaStream_t stream) {
-    const dim3 grid(blocks), block(warps * 32);
-    switch (mode) {
-        case kModeEngine: ant_kernel<kModeEngine><<<grid, block, smem, stream>>>(L); break;
-        case kModeVisits: ant_kernel<kModeVisits><<<grid, block, smem, stream>>>(L); break;
-        case kModeUniforms: ant_kernel<kModeUniforms><<<grid, block, smem, stream>>>(L); break;
-        case kModePrepare: ant_kernel<kModePrepare><<<grid, block, smem, stream>>>(L); break;
-        case kModeEngineGlobal: ant_kernel<kModeEngineGlobal><<<grid, block, smem, stream>>>(L); break;
-        case kModeEngineFollow: ant_kernel<kModeEngineFollow><<<grid, block, smem, stream>>>(L); break;
-        case kModeEngineGlobalFollow: ant_kernel<kModeEngineGlobalFollow><<<grid, block, smem, stream>>>(L); break;
-        case kModeEngineFollowDense: ant_kernel<kModeEngineFollowDense><<<grid, block, smem, stream>>>(L); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
+    return for_variant(mode, L.ls_mode, [&](auto m) {
+        ant_kernel<decltype(m)::value><<<dim3(blocks), dim3(warps * 32), smem, stream>>>(L);
+        return cudaGetLastError();
+    });
 }
 
 // ---------------------------------------------------------------------------

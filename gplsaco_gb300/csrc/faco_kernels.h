@@ -20,9 +20,11 @@ namespace faco {
 // 68.9 / 72.5 / 78.5 / 79.8 ms; 32 x 128 ants at N=537 27.1 / 27.7 / 29.3 /
 // 30.1 / 29.9 ms; one N=100 colony 4.80 / 4.79 / 5.01 / 5.20 / 5.25 ms; the
 // large panel (global-memory workspace, 2-opt) 497 / 504 / 529 / 542 / 542 ms.
+// With Or-opt (more registers) full panels too run 5: 256 x 32 ants at N=1000,
+// 160 iterations, 5 / 6 / 7 blocks: 71.0 / 73.3 / 74.9 ms.
 constexpr std::uint32_t kMaxWarpsPerBlock = 4;
 constexpr std::uint32_t ant_blocks_per_sm(int mode) {
-    return dense_mode(mode) ? 7 : global_mode(mode) ? 4 : follow_mode(mode) ? 5 : 6;
+    return dense_mode(mode) ? (mode & kOrOptOnly ? 5 : 7) : global_mode(mode) || !engine_mode(mode) ? 4 : 5;
 }
 
 struct ColonyParams {
@@ -53,7 +55,7 @@ cudaError_t launch_knn(const int2* xy, std::uint32_t n, std::uint32_t needed, no
                        std::int32_t* near_dist, cudaStream_t stream);
 
 // Host-side launchers (the kernels are defined in faco_kernels.cu).
-cudaError_t prepare_ant_kernel(int mode, std::uint32_t smem_bytes);
+cudaError_t prepare_ant_kernel(int mode, std::uint32_t ls_mode, std::uint32_t smem_bytes);
 cudaError_t launch_ant_kernel(int mode, const AntLaunch& L, std::uint32_t blocks, std::uint32_t warps,
                               std::uint32_t smem_bytes, cudaStream_t stream);
 
