@@ -19,6 +19,7 @@ enum DeviceError : unsigned {
     kErrLoopCap = 1u << 2,
     kErrShape = 1u << 3,
     kErrTensorWait = 1u << 4,   // a tcgen05 MMA completion wait ran out
+    kErrFeature = 1u << 5,      // a controller feature outside [0, 1]
 };
 
 // TSPLIB EUC_2D: round(sqrt(dx^2+dy^2)) with halves up.  sqrt(s) is never a

@@ -1795,6 +1795,78 @@ int faco_validate_program(const faco_program* p) {
     });
 }
 
+}  // extern "C"
+
+namespace {
+
+// The device side of one scoring call: every buffer a slice of one
+// allocation (a call of five allocations and frees spends more on them than
+// on the kernel).
+struct ScoreCall {
+    cudaStream_t stream = nullptr;
+    std::uint32_t blocks = 0;
+    unsigned char* programs = nullptr;
+    std::uint32_t* kinds = nullptr;
+    float* features = nullptr;
+    std::uint32_t* masks = nullptr;
+    float* scores = nullptr;
+    std::int32_t* actions = nullptr;
+    unsigned* error = nullptr;
+    void upload(void* to, const void* from, std::size_t bytes) const {
+        cuda_check(cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, stream), "upload");
+    }
+};
+
+// Uploads the features and masks, runs `launch` (which uploads the programs)
+// and, where every feature was in [0, 1] and every mask legal, downloads the
+// scores and actions; nothing is written to them otherwise.
+template <class Launch>
+void score_on_device(const float* features, const std::uint32_t* masks, std::uint32_t colonies, float* scores,
+                     std::int32_t* actions, std::size_t program_bytes, std::uint32_t kinds, Launch&& launch) {
+    const std::size_t feature_bytes = 12ull * colonies * 32 * sizeof(float), score_bytes = colonies * 32ull * sizeof(float);
+    std::size_t total = 0;
+    const auto slice = [&](std::size_t bytes) {
+        const std::size_t at = total;
+        total += (bytes + 255) & ~std::size_t{255};
+        return at;
+    };
+    const std::size_t at_error = slice(sizeof(unsigned)), at_programs = slice(program_bytes),
+                      at_kinds = slice(kinds * sizeof(std::uint32_t)), at_masks = slice(colonies * sizeof(std::uint32_t)),
+                      at_actions = slice(colonies * sizeof(std::int32_t)), at_scores = slice(score_bytes),
+                      at_features = slice(feature_bytes);
+    DeviceBuffer<unsigned char> buffer(total);
+    unsigned char* base = buffer.get();
+    ScoreCall d;
+    d.blocks = (colonies + 3) / 4;
+    d.error = reinterpret_cast<unsigned*>(base + at_error);
+    d.programs = base + at_programs;
+    d.kinds = reinterpret_cast<std::uint32_t*>(base + at_kinds);
+    d.masks = reinterpret_cast<std::uint32_t*>(base + at_masks);
+    d.actions = reinterpret_cast<std::int32_t*>(base + at_actions);
+    d.scores = reinterpret_cast<float*>(base + at_scores);
+    d.features = reinterpret_cast<float*>(base + at_features);
+    cuda_check(cudaMemsetAsync(d.error, 0, sizeof(unsigned), d.stream), "memset");
+    d.upload(d.features, features, feature_bytes);
+    d.upload(d.masks, masks, colonies * sizeof(std::uint32_t));
+    launch(d);
+    cuda_check(cudaGetLastError(), "score launch");
+    bool legal = true;
+    for (std::uint32_t c = 0; c < colonies; ++c) legal = legal && masks[c] != 0;
+    unsigned error = 0;
+    cuda_check(cudaMemcpyAsync(&error, d.error, sizeof error, cudaMemcpyDeviceToHost, d.stream), "download");
+    cuda_check(cudaStreamSynchronize(d.stream), "score");
+    require(!error, "features must be finite and in [0, 1]");
+    require(legal, "a colony has no legal action");
+    cuda_check(cudaMemcpyAsync(scores, d.scores, score_bytes, cudaMemcpyDeviceToHost, d.stream), "download");
+    cuda_check(cudaMemcpyAsync(actions, d.actions, colonies * sizeof(std::int32_t), cudaMemcpyDeviceToHost, d.stream),
+               "download");
+    cuda_check(cudaStreamSynchronize(d.stream), "score");
+}
+
+}  // namespace
+
+extern "C" {
+
 int faco_score(const faco_program* programs, uint32_t n_programs, const float* features, uint32_t features_count,
                const uint32_t* masks, uint32_t colonies, float* scores, int32_t* actions) {
     return guarded([&] {
@@ -1804,29 +1876,14 @@ int faco_score(const faco_program* programs, uint32_t n_programs, const float* f
         require(features_count == 12, "features must be [12, colonies, 32]");
         for (std::uint32_t i = 0; i < n_programs; ++i)
             if (faco_validate_program(programs + i) != FACO_OK) throw Error(FACO_EINVAL, g_error);
-        const std::size_t nf = static_cast<std::size_t>(features_count) * colonies * 32;
-        for (std::size_t i = 0; i < nf; ++i)
-            require(std::isfinite(features[i]) && features[i] >= 0.0f && features[i] <= 1.0f,
-                    "features must be finite and in [0, 1]");
-        for (std::uint32_t c = 0; c < colonies; ++c) require(masks[c] != 0, "a colony has no legal action");
         static_assert(sizeof(faco::Program) == sizeof(faco_program), "program layout");
-        DeviceBuffer<faco::Program> d_prog;
-        DeviceBuffer<float> d_feat, d_scores;
-        DeviceBuffer<std::uint32_t> d_masks;
-        DeviceBuffer<std::int32_t> d_actions;
-        cudaStream_t s = nullptr;
-        d_prog.upload(reinterpret_cast<const faco::Program*>(programs), n_programs, s);
-        d_feat.upload(features, nf, s);
-        d_masks.upload(masks, colonies, s);
-        d_scores.resize(static_cast<std::size_t>(colonies) * 32);
-        d_actions.resize(colonies);
-        const std::uint32_t blocks = (colonies * 32 + 127) / 128;
-        faco::score_kernel<<<blocks, 128, 0, s>>>(d_prog.get(), colonies / n_programs, d_feat.get(), d_masks.get(),
-                                                  d_scores.get(), d_actions.get(), colonies);
-        cuda_check(cudaGetLastError(), "score launch");
-        d_scores.download(scores, static_cast<std::size_t>(colonies) * 32, s);
-        d_actions.download(actions, colonies, s);
-        cuda_check(cudaStreamSynchronize(s), "score");
+        score_on_device(features, masks, colonies, scores, actions, n_programs * sizeof(faco_program), 0,
+                        [&](const ScoreCall& d) {
+                            d.upload(d.programs, programs, n_programs * sizeof(faco_program));
+                            faco::score_kernel<<<d.blocks, 128, 0, d.stream>>>(
+                                reinterpret_cast<const faco::Program*>(d.programs), colonies / n_programs, d.features,
+                                d.masks, d.scores, d.actions, colonies, d.error);
+                        });
     });
 }
 
@@ -1839,31 +1896,17 @@ int faco_score_controllers(const faco_program* trees, const uint32_t* kinds, uin
                 "colonies must be a multiple of the controller count");
         require(features_count == 12, "features must be [12, colonies, 32]");
         for (std::uint32_t i = 0; i < n_controllers; ++i) validate_controller(trees + 3ull * i, kinds[i]);
-        const std::size_t nf = static_cast<std::size_t>(features_count) * colonies * 32;
-        for (std::size_t i = 0; i < nf; ++i)
-            require(std::isfinite(features[i]) && features[i] >= 0.0f && features[i] <= 1.0f,
-                    "features must be finite and in [0, 1]");
-        for (std::uint32_t c = 0; c < colonies; ++c) require(masks[c] != 0, "a colony has no legal action");
-        DeviceBuffer<faco::Program> d_trees;
-        DeviceBuffer<std::uint32_t> d_kinds, d_masks;
-        DeviceBuffer<float> d_feat, d_scores;
-        DeviceBuffer<std::int32_t> d_actions;
-        cudaStream_t s = nullptr;
-        d_trees.upload(reinterpret_cast<const faco::Program*>(trees), 3ull * n_controllers, s);
-        d_kinds.upload(kinds, n_controllers, s);
-        d_feat.upload(features, nf, s);
-        d_masks.upload(masks, colonies, s);
-        d_scores.resize(static_cast<std::size_t>(colonies) * 32);
-        cuda_check(cudaMemsetAsync(d_scores.get(), 0, static_cast<std::size_t>(colonies) * 32 * sizeof(float), s),
-                   "memset");
-        d_actions.resize(colonies);
-        faco::score_controllers_kernel<<<(colonies * 32 + 127) / 128, 128, 0, s>>>(
-            d_trees.get(), d_kinds.get(), colonies / n_controllers, d_feat.get(), d_masks.get(), d_scores.get(),
-            d_actions.get(), colonies);
-        cuda_check(cudaGetLastError(), "score launch");
-        d_scores.download(scores, static_cast<std::size_t>(colonies) * 32, s);
-        d_actions.download(actions, colonies, s);
-        cuda_check(cudaStreamSynchronize(s), "score");
+        const std::size_t tree_bytes = 3ull * n_controllers * sizeof(faco_program);
+        score_on_device(features, masks, colonies, scores, actions, tree_bytes, n_controllers,
+                        [&](const ScoreCall& d) {
+                            d.upload(d.programs, trees, tree_bytes);
+                            d.upload(d.kinds, kinds, n_controllers * sizeof(std::uint32_t));
+                            cuda_check(cudaMemsetAsync(d.scores, 0, colonies * 32ull * sizeof(float), d.stream),
+                                       "memset");
+                            faco::score_controllers_kernel<<<d.blocks, 128, 0, d.stream>>>(
+                                reinterpret_cast<const faco::Program*>(d.programs), d.kinds, colonies / n_controllers,
+                                d.features, d.masks, d.scores, d.actions, colonies, d.error);
+                        });
     });
 }
 
