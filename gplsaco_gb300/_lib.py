@@ -29,7 +29,7 @@ EXPORTED = (
     "faco_register_problem", "faco_problem_rows", "faco_evaluate", "faco_validate_program", "faco_score",
     "faco_ant_diagnostic", "faco_pheromone_step", "faco_begin", "faco_step", "faco_step_timed", "faco_finish",
     "faco_engine_stream", "faco_evaluate_programs", "faco_mlp_param_count", "faco_mlp_forward", "faco_mlp_gradient",
-    "faco_mlp_train", "faco_edge_data", "faco_prior_set", "faco_prior_refresh", "faco_current_costs",
+    "faco_mlp_train", "faco_mlp_train_order", "faco_edge_data", "faco_prior_set", "faco_prior_refresh", "faco_current_costs",
     "faco_colony_rows",
     "faco_set_mne_targets", "faco_get_launch_plan",
     "faco_pheromone_step_noalloc", "faco_begin_programs", "faco_snapshot", "faco_restore",
@@ -155,6 +155,7 @@ def load():
     L.faco_mlp_forward.argtypes = [vp, vp, C.c_uint32, vp]
     L.faco_mlp_gradient.argtypes = [vp, vp, vp, C.c_uint32, vp, vp]
     L.faco_mlp_train.argtypes = [vp, vp, vp, C.c_uint32, C.c_uint32, C.c_uint32, C.c_float, vp]
+    L.faco_mlp_train_order.argtypes = [vp, vp, vp, vp, C.c_uint32, C.c_uint32, C.c_uint32, C.c_float, vp]
     L.faco_edge_data.argtypes = [vp, vp, vp, C.c_uint64, C.POINTER(C.c_uint64)]
     L.faco_prior_set.argtypes = [vp, vp, C.c_float, C.c_int, vp, C.c_uint32]
     L.faco_prior_refresh.argtypes = [vp]

@@ -249,6 +249,24 @@ std::vector<std::uint32_t> parent_neighbours(const std::uint32_t* tour, std::uin
     return nbr;
 }
 
+// Launches a kernel that waits on the device for the kernel before it on the
+// stream (programmatic dependent launch).
+template <class... Params, class... Args>
+void launch_dependent(void (*kernel)(Params...), std::uint32_t blocks, std::uint32_t threads, std::uint32_t smem,
+                             cudaStream_t s, Args... args) {
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(blocks);
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = smem;
+    config.stream = s;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    cuda_check(cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...), "training step");
+}
+
 void launch_ants(int mode, const faco::AntLaunch& L, std::uint32_t blocks, std::uint32_t warps, cudaStream_t s) {
     const std::uint32_t smem = faco::block_smem_bytes(L.n_max, warps);
     cuda_check(faco::prepare_ant_kernel(mode, L.ls_mode, smem), "cudaFuncSetAttribute");
@@ -2200,57 +2218,86 @@ int faco_mlp_gradient(const float* params, const uint16_t* x, const float* y, ui
     });
 }
 
+static void train_mlp(float* params, const uint16_t* x, const float* y, const uint32_t* order, uint32_t count,
+                      uint32_t epochs, uint32_t batch, float lr, float* epoch_losses) {
+    cudaStream_t s = nullptr;
+    DeviceBuffer<faco::MlpParams> P, M, V;
+    DeviceBuffer<faco::MlpOperands> O;
+    upload_mlp(P, O, params, s);
+    M.resize(1); V.resize(1);
+    cuda_check(cudaMemsetAsync(M.get(), 0, sizeof(faco::MlpParams), s), "memset");
+    cuda_check(cudaMemsetAsync(V.get(), 0, sizeof(faco::MlpParams), s), "memset");
+    DeviceBuffer<__nv_bfloat16> dx, x_raw;
+    DeviceBuffer<float> dy, y_raw, dl(epochs);
+    DeviceBuffer<std::uint32_t> d_order;
+    const std::size_t values = static_cast<std::size_t>(count) * faco::kMlpIn;
+    (order ? x_raw : dx).upload(reinterpret_cast<const __nv_bfloat16*>(x), values, s);
+    (order ? y_raw : dy).upload(y, count, s);
+    if (order) {
+        d_order.upload(order, count, s);
+        dx.resize(values);
+        dy.resize(count);
+        faco::gather_rows_kernel<<<std::min((count + 255) / 256, 1216u), 256, 0, s>>>(
+            reinterpret_cast<const uint4*>(x_raw.get()), y_raw.get(), d_order.get(), count,
+            reinterpret_cast<uint4*>(dx.get()), dy.get());
+        cuda_check(cudaGetLastError(), "row order");
+    }
+    cuda_check(cudaMemsetAsync(dl.get(), 0, sizeof(float) * epochs, s), "memset");
+    const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
+    std::uint64_t step = 0;
+    cuda_check(prepare_tensor_kernels(), "tcgen05 kernel attributes");
+    const std::uint32_t max_blocks = grad_blocks(std::min(batch, count));
+    DeviceBuffer<faco::MlpParams> partials(max_blocks);
+    DeviceBuffer<float> loss_partials(max_blocks);
+    DeviceBuffer<unsigned> derr(1);
+    cuda_check(cudaMemsetAsync(derr.get(), 0, sizeof(unsigned), s), "memset");
+    constexpr std::uint32_t kStepBlocks = (faco::kMlpParamCount + 1 + 127) / 128;
+    for (std::uint32_t ep = 0; ep < epochs; ++ep) {
+        for (std::uint32_t first = 0; first < count;) {
+            const std::uint32_t size = std::min(batch, count - first);
+            const std::uint32_t blocks = grad_blocks(size);
+            ++step;
+            // both wait on the device for the kernel before them, so the
+            // next one's launch and prologue overlap it
+            launch_dependent(faco::mlp_grad_kernel, blocks, 128, faco::tc::kGradSmemBytes, s, P.get(), O.get(),
+                             dx.get() + static_cast<std::size_t>(first) * faco::kMlpIn, dy.get() + first, size,
+                             1.0f / size, partials.get(), loss_partials.get(), derr.get());
+            const float b1 = 1.0f - std::pow(beta1, static_cast<float>(step));
+            const float b2 = 1.0f - std::pow(beta2, static_cast<float>(step));
+            launch_dependent(faco::mlp_step_kernel, kStepBlocks, 128, 0, s, partials.get(), loss_partials.get(),
+                             blocks, P.get(), O.get(), M.get(), V.get(), lr, beta1, beta2, eps, b1, b2,
+                             dl.get() + ep);
+            first += size;
+        }
+    }
+    std::vector<float> losses(epochs);
+    dl.download(losses.data(), epochs, s);
+    unsigned err = 0;
+    derr.download(&err, 1, s);
+    cuda_check(cudaStreamSynchronize(s), "mlp training");
+    if (err) throw Error(FACO_EDEVICE, "device error word " + std::to_string(err) + " in the MLP gradient");
+    P.download(reinterpret_cast<faco::MlpParams*>(params), 1, s);
+    cuda_check(cudaStreamSynchronize(s), "mlp training");
+    if (epoch_losses)
+        for (std::uint32_t ep = 0; ep < epochs; ++ep) epoch_losses[ep] = losses[ep] / count;
+}
+
 int faco_mlp_train(float* params, const uint16_t* x, const float* y, uint32_t count, uint32_t epochs,
                    uint32_t batch, float lr, float* epoch_losses) {
     return guarded([&] {
         require(params && x && y && count > 0 && batch > 0 && epochs > 0 && lr > 0, "invalid arguments");
-        cudaStream_t s = nullptr;
-        DeviceBuffer<faco::MlpParams> P, G, M, V;
-        DeviceBuffer<faco::MlpOperands> O;
-        upload_mlp(P, O, params, s);
-        G.resize(1); M.resize(1); V.resize(1);
-        cuda_check(cudaMemsetAsync(M.get(), 0, sizeof(faco::MlpParams), s), "memset");
-        cuda_check(cudaMemsetAsync(V.get(), 0, sizeof(faco::MlpParams), s), "memset");
-        DeviceBuffer<__nv_bfloat16> dx;
-        dx.upload(reinterpret_cast<const __nv_bfloat16*>(x), static_cast<std::size_t>(count) * faco::kMlpIn, s);
-        DeviceBuffer<float> dy, dl(epochs);
-        dy.upload(y, count, s);
-        cuda_check(cudaMemsetAsync(dl.get(), 0, sizeof(float) * epochs, s), "memset");
-        const float beta1 = 0.9f, beta2 = 0.999f, eps = 1e-8f;
-        std::uint64_t step = 0;
-        cuda_check(prepare_tensor_kernels(), "tcgen05 kernel attributes");
-        const std::uint32_t max_blocks = grad_blocks(std::min(batch, count));
-        DeviceBuffer<faco::MlpParams> partials(max_blocks);
-        DeviceBuffer<float> loss_partials(max_blocks);
-        DeviceBuffer<unsigned> derr(1);
-        cuda_check(cudaMemsetAsync(derr.get(), 0, sizeof(unsigned), s), "memset");
-        for (std::uint32_t ep = 0; ep < epochs; ++ep) {
-            for (std::uint32_t first = 0; first < count; first += batch) {
-                const std::uint32_t size = std::min(batch, count - first);
-                const std::uint32_t blocks = grad_blocks(size);
-                ++step;
-                faco::mlp_grad_kernel<<<blocks, 128, faco::tc::kGradSmemBytes, s>>>(
-                    P.get(), O.get(), dx.get() + static_cast<std::size_t>(first) * faco::kMlpIn, dy.get() + first,
-                    size, 1.0f / size, partials.get(), loss_partials.get(), derr.get());
-                faco::mlp_grad_reduce_kernel<<<20, 256, 0, s>>>(partials.get(), loss_partials.get(), blocks, G.get(),
-                                                                dl.get() + ep);
-                const float b1 = 1.0f - std::pow(beta1, static_cast<float>(step));
-                const float b2 = 1.0f - std::pow(beta2, static_cast<float>(step));
-                faco::adam_kernel<<<20, 256, 0, s>>>(P.get(), G.get(), M.get(), V.get(), lr, beta1, beta2, eps, b1, b2);
-                faco::refresh_operands_kernel<<<4, 256, 0, s>>>(P.get(), O.get());
-                cuda_check(cudaGetLastError(), "training step");
-            }
-        }
-        std::vector<float> losses(epochs);
-        dl.download(losses.data(), epochs, s);
-        unsigned err = 0;
-        derr.download(&err, 1, s);
-        cuda_check(cudaStreamSynchronize(s), "mlp training");
-        if (err) throw Error(FACO_EDEVICE, "device error word " + std::to_string(err) + " in the MLP gradient");
-        P.download(reinterpret_cast<faco::MlpParams*>(params), 1, s);
-        cuda_check(cudaStreamSynchronize(s), "mlp training");
-        if (epoch_losses)
-            for (std::uint32_t ep = 0; ep < epochs; ++ep) epoch_losses[ep] = losses[ep] / count;
+        train_mlp(params, x, y, nullptr, count, epochs, batch, lr, epoch_losses);
+    });
+}
+
+int faco_mlp_train_order(float* params, const uint16_t* x, const float* y, const uint32_t* order, uint32_t count,
+                         uint32_t epochs, uint32_t batch, float lr, float* epoch_losses) {
+    return guarded([&] {
+        require(params && x && y && order && count > 0 && batch > 0 && epochs > 0 && lr > 0, "invalid arguments");
+        std::uint32_t largest = 0;
+        for (std::uint32_t i = 0; i < count; ++i) largest = std::max(largest, order[i]);
+        require(largest < count, "row order out of range");
+        train_mlp(params, x, y, order, count, epochs, batch, lr, epoch_losses);
     });
 }
 

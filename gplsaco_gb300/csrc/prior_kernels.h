@@ -19,8 +19,11 @@ __global__ void mlp_grad_kernel(const MlpParams* P, const MlpOperands* O, const 
                                 unsigned* error);
 __global__ void mlp_grad_reduce_kernel(const MlpParams* partials, const float* loss_partials, std::uint32_t blocks,
                                        MlpParams* grad, float* loss);
-__global__ void adam_kernel(MlpParams* P, const MlpParams* grad, MlpParams* m, MlpParams* v, float lr, float beta1,
-                            float beta2, float eps, float bias1, float bias2);
+__global__ void mlp_step_kernel(const MlpParams* partials, const float* loss_partials, std::uint32_t blocks,
+                                MlpParams* P, MlpOperands* O, MlpParams* m, MlpParams* v, float lr, float beta1,
+                                float beta2, float eps, float bias1, float bias2, float* loss);
+__global__ void gather_rows_kernel(const uint4* x, const float* y, const std::uint32_t* order, std::uint32_t count,
+                                   uint4* x_out, float* y_out);
 __global__ void refresh_operands_kernel(const MlpParams* P, MlpOperands* O);
 __global__ void edge_features_kernel(const InstanceView* instances, const ColonyView* colonies,
                                      const ColonyState* states, std::uint32_t first, const std::uint64_t* row_offset,

@@ -1,6 +1,8 @@
 // prior_mlp.cu -- forward, backward and Adam kernels of the edge-prior MLP.
 #include <cuda_runtime.h>
 
+#include <cstddef>
+
 #include "prior_kernels.h"
 #include "prior_mlp.cuh"
 #include "prior_mlp_tc.cuh"
@@ -37,6 +39,7 @@ __global__ void __launch_bounds__(128) mlp_grad_kernel(const MlpParams* P, const
                                                        float inv_count, MlpParams* partials, float* loss_partials,
                                                        unsigned* error) {
     extern __shared__ __align__(16) unsigned char smem[];
+    tc::start_next_kernel();
     tc::gradient_rows(
         P, O, E, inv_count, smem, error,
         [&](std::uint32_t row) { return *reinterpret_cast<const uint4*>(x + (size_t)row * kMlpIn); },
@@ -60,18 +63,64 @@ __global__ void mlp_grad_reduce_kernel(const MlpParams* partials, const float* l
     }
 }
 
-// Adam on the FP32 masters (decoupled from the BF16 operand refresh below).
-__global__ void adam_kernel(MlpParams* P, const MlpParams* grad, MlpParams* m, MlpParams* v, float lr, float beta1,
-                            float beta2, float eps, float bias1, float bias2) {
+// x[0] + x[stride] + ... (count values, in that order, from zero), 32 loads in
+// flight.
+__device__ __forceinline__ float ordered_sum(const float* x, std::size_t stride, std::uint32_t count) {
+    constexpr std::uint32_t kAhead = 32;
+    float sum = 0.f;
+    std::uint32_t b = 0;
+    for (; b + kAhead <= count; b += kAhead) {
+        float t[kAhead];
+#pragma unroll
+        for (std::uint32_t u = 0; u < kAhead; ++u) t[u] = x[(b + u) * stride];
+#pragma unroll
+        for (std::uint32_t u = 0; u < kAhead; ++u) sum += t[u];
+    }
+    for (; b < count; ++b) sum += x[b * stride];
+    return sum;
+}
+
+// One training step after the gradient: per parameter the block partials
+// summed in block order, Adam on the FP32 master, and its BF16 operand copy;
+// *loss += the step's losses.  One thread per parameter (and one for the
+// loss), one launch.  Bound by latency, as the gradient of one 8,192-row batch
+// is (64 CTAs of one tile): with three kernels after the gradient, scalar
+// weight loads and stores in it and plain launches a step took 31 us, now 13.
+__global__ void __launch_bounds__(128) mlp_step_kernel(const MlpParams* partials, const float* loss_partials,
+                                                       std::uint32_t blocks, MlpParams* P, MlpOperands* O,
+                                                       MlpParams* m, MlpParams* v, float lr, float beta1, float beta2,
+                                                       float eps, float bias1, float bias2, float* loss) {
+    tc::start_next_kernel();
+    tc::wait_previous_kernel();
+    const float* src = reinterpret_cast<const float*>(partials);
     float* p = reinterpret_cast<float*>(P);
-    const float* gr = reinterpret_cast<const float*>(grad);
     float* mm = reinterpret_cast<float*>(m);
     float* vv = reinterpret_cast<float*>(v);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kMlpParamCount; i += gridDim.x * blockDim.x) {
-        const float gi = gr[i];
-        mm[i] = beta1 * mm[i] + (1.0f - beta1) * gi;
-        vv[i] = beta2 * vv[i] + (1.0f - beta2) * gi * gi;
-        p[i] -= lr * (mm[i] / bias1) / (sqrtf(vv[i] / bias2) + eps);
+    constexpr int kW2 = offsetof(MlpParams, w2) / sizeof(float);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < kMlpParamCount) {
+        const float m0 = mm[i], v0 = vv[i], p0 = p[i];
+        const float gi = ordered_sum(src + i, kMlpParamCount, blocks);
+        const float m1 = beta1 * m0 + (1.0f - beta1) * gi;
+        const float v1 = beta2 * v0 + (1.0f - beta2) * gi * gi;
+        const float p1 = p0 - lr * (m1 / bias1) / (sqrtf(v1 / bias2) + eps);
+        mm[i] = m1;
+        vv[i] = v1;
+        p[i] = p1;
+        if (i < kMlpHidden * kMlpIn) O->w1[i] = __float2bfloat16(p1);
+        else if (i >= kW2 && i < kW2 + kMlpHidden * kMlpHidden) O->w2[i - kW2] = __float2bfloat16(p1);
+    } else if (i == kMlpParamCount) {
+        *loss += ordered_sum(loss_partials, 1, blocks);
+    }
+}
+
+// Rows of x ([count][8] BF16, 16 bytes) and y taken in `order`.
+__global__ void gather_rows_kernel(const uint4* x, const float* y, const std::uint32_t* order, std::uint32_t count,
+                                   uint4* x_out, float* y_out) {
+    for (std::uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        const std::uint32_t r = order[i];
+        x_out[i] = x[r];
+        y_out[i] = y[r];
     }
 }
 

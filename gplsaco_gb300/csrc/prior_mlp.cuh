@@ -28,12 +28,13 @@ struct MlpParams {
     float pad[3];
 };
 
-struct MlpOperands {
+struct alignas(16) MlpOperands {   // read 16 bytes at a time
     __nv_bfloat16 w1[kMlpHidden * kMlpIn];          // [out][in]
     __nv_bfloat16 w2[kMlpHidden * kMlpHidden];      // [out][in]
 };
 
 constexpr int kMlpParamCount = sizeof(MlpParams) / sizeof(float);
+static_assert(sizeof(MlpParams) % 16 == 0, "arrays of parameters keep 16-byte alignment");
 
 __device__ __forceinline__ std::uint32_t pack_bf16(float lo, float hi) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);

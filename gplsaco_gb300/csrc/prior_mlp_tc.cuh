@@ -142,17 +142,15 @@ __device__ bool forward_rows(const MlpParams* P, const MlpOperands* O, std::uint
     unsigned char* hs = xs + kXBytes;
     unsigned char* w1s = hs + kHBytes;
     unsigned char* w2s = w1s + kW1Bytes;
-    // weights as B operands (N = 64 rows = output units, K-major); W1's K
-    // padded from 8 to 16 with zeros
-    for (std::uint32_t i = tid; i < 64 * 16; i += blockDim.x) {
-        const std::uint32_t n = i >> 4, k = i & 15u;
-        const __nv_bfloat16 v = k < kMlpIn ? O->w1[n * kMlpIn + k] : __float2bfloat16(0.0f);
-        *reinterpret_cast<__nv_bfloat16*>(w1s + operand_offset(n, k, 64)) = v;
+    // weights as B operands (N = 64 rows = output units, K-major), eight
+    // inputs per 16-byte copy; W1's K padded from 8 to 16 with zeros
+    for (std::uint32_t n = tid; n < 64; n += blockDim.x) {
+        *reinterpret_cast<uint4*>(w1s + operand_offset(n, 0, 64)) = reinterpret_cast<const uint4*>(O->w1)[n];
+        *reinterpret_cast<uint4*>(w1s + operand_offset(n, 8, 64)) = make_uint4(0, 0, 0, 0);
     }
-    for (std::uint32_t i = tid; i < 64 * 64; i += blockDim.x) {
-        const std::uint32_t n = i >> 6, k = i & 63u;
-        *reinterpret_cast<__nv_bfloat16*>(w2s + operand_offset(n, k, 64)) = O->w2[n * 64 + k];
-    }
+    for (std::uint32_t i = tid; i < 64 * 8; i += blockDim.x)
+        *reinterpret_cast<uint4*>(w2s + operand_offset(i >> 3, (i & 7u) * 8, 64)) =
+            reinterpret_cast<const uint4*>(O->w2)[i];
     for (std::uint32_t i = tid; i < 64; i += blockDim.x) {
         s_b1[i] = P->b1[i];
         s_b2[i] = P->b2[i];
@@ -332,6 +330,12 @@ __device__ __forceinline__ uint4 pack8(const float* a) {
     return make_uint4(pack_bf16(a[0], a[1]), pack_bf16(a[2], a[3]), pack_bf16(a[4], a[5]), pack_bf16(a[6], a[7]));
 }
 
+// Programmatic dependent launch: lets the next kernel of the stream start its
+// prologue now; waits until the previous one is complete and its writes are
+// visible (both without effect in an ordinary launch).
+__device__ __forceinline__ void start_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Partial gradient and loss sum of this CTA's rows (128-row tiles strided
 // over the grid) into *grad and *loss_sum.  128 threads, `smem` holds
 // kGradSmemBytes (16-byte aligned).  Returns false (and sets
@@ -346,21 +350,7 @@ __device__ bool gradient_rows(const MlpParams* P, const MlpOperands* O, std::uin
     __shared__ __align__(16) float s_b1[64], s_b2[64], s_w3[64];
     __shared__ float s_scalar[4][2];
     const std::uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    for (std::uint32_t i = tid; i < 64 * 16; i += blockDim.x) {
-        const std::uint32_t o = i >> 4, f = i & 15u;
-        const __nv_bfloat16 v = f < kMlpIn ? O->w1[o * kMlpIn + f] : __float2bfloat16(0.0f);
-        *reinterpret_cast<__nv_bfloat16*>(smem + kGradW1 + weight_offset(o, f)) = v;
-    }
-    for (std::uint32_t i = tid; i < 64 * 64; i += blockDim.x) {
-        const std::uint32_t o = i >> 6, f = i & 63u;
-        *reinterpret_cast<__nv_bfloat16*>(smem + kGradW2 + weight_offset(o, f)) = O->w2[o * 64 + f];
-    }
-    for (std::uint32_t i = tid; i < 64; i += blockDim.x) {
-        s_b1[i] = P->b1[i];
-        s_b2[i] = P->b2[i];
-        s_w3[i] = P->w3[i];
-    }
-    const float b3 = P->b3;
+    // what needs nothing of the previous kernel comes before the wait for it
     if (tid == 0) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&bar)) : "memory");
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
@@ -368,6 +358,37 @@ __device__ bool gradient_rows(const MlpParams* P, const MlpOperands* O, std::uin
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    wait_previous_kernel();
+    // weights, biases and this thread's first row: every load before the
+    // first store that waits for one (128 threads); read one after the other
+    // they took 3,100 of a one-tile CTA's 11,500 cycles
+    uint4 w1v = make_uint4(0, 0, 0, 0), w2v[4], v = make_uint4(0, 0, 0, 0);
+    float b1v = 0.f, b2v = 0.f, w3v = 0.f, y = 0.f;
+    if (tid < 64) {
+        w1v = reinterpret_cast<const uint4*>(O->w1)[tid];
+        b1v = P->b1[tid];
+        b2v = P->b2[tid];
+        w3v = P->w3[tid];
+    }
+#pragma unroll
+    for (std::uint32_t u = 0; u < 4; ++u) w2v[u] = reinterpret_cast<const uint4*>(O->w2)[tid + 128 * u];
+    if (blockIdx.x * kRows + tid < count) {
+        v = feat(blockIdx.x * kRows + tid);
+        y = label(blockIdx.x * kRows + tid);
+    }
+    if (tid < 64) {
+        *reinterpret_cast<uint4*>(smem + kGradW1 + weight_offset(tid, 0)) = w1v;
+        *reinterpret_cast<uint4*>(smem + kGradW1 + weight_offset(tid, 8)) = make_uint4(0, 0, 0, 0);
+        s_b1[tid] = b1v;
+        s_b2[tid] = b2v;
+        s_w3[tid] = w3v;
+    }
+#pragma unroll
+    for (std::uint32_t u = 0; u < 4; ++u) {
+        const std::uint32_t i = tid + 128 * u;
+        *reinterpret_cast<uint4*>(smem + kGradW2 + weight_offset(i >> 3, (i & 7u) * 8)) = w2v[u];
+    }
+    const float b3 = P->b3;
     fence_before();
     __syncthreads();
     fence_after();
@@ -380,12 +401,6 @@ __device__ bool gradient_rows(const MlpParams* P, const MlpOperands* O, std::uin
     bool ok = true, any = false;
     float db3 = 0.f, lsum = 0.f;
     const std::uint32_t stride = gridDim.x * kRows;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    float y = 0.f;
-    if (blockIdx.x * kRows + tid < count) {
-        v = feat(blockIdx.x * kRows + tid);
-        y = label(blockIdx.x * kRows + tid);
-    }
     for (std::uint32_t first = blockIdx.x * kRows; first < count; first += stride) {
         const std::uint32_t row = first + tid;
         const bool valid = row < count;
@@ -540,7 +555,9 @@ __device__ bool gradient_rows(const MlpParams* P, const MlpOperands* O, std::uin
             for (std::uint32_t c = 0; c < 64; c += 16) {
                 load16(tmem + lane_base + kGradColGW + c, a);
 #pragma unroll
-                for (int t = 0; t < 16; ++t) grad->w2[o * 64 + c + t] = any ? a[t] : 0.f;
+                for (int t = 0; t < 16; t += 4)   // (every partial starts on 16 bytes)
+                    *reinterpret_cast<float4*>(grad->w2 + o * 64 + c + t) =
+                        any ? make_float4(a[t], a[t + 1], a[t + 2], a[t + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
             load16(tmem + lane_base + kGradColGW + 64, a);
             grad->b2[o] = any ? a[8] : 0.f;

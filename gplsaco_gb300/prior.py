@@ -79,15 +79,16 @@ def gradient(params: np.ndarray, x_bits: np.ndarray, y: np.ndarray):
 
 def train(params: np.ndarray, x_bits: np.ndarray, y: np.ndarray, *, epochs: int = 10, batch: int = 8192,
           lr: float = 2e-3, seed: int = 0):
-    """Adam on the GPU; rows are shuffled once on the host (seeded)."""
+    """Adam on the GPU over the rows in one seeded random order."""
     params = np.array(params, np.float32, copy=True)
     x_bits = np.ascontiguousarray(x_bits, np.uint16).reshape(-1, IN)
     y = np.ascontiguousarray(y, np.float32)
-    order = np.random.default_rng(seed).permutation(y.size)
-    xs, ys = np.ascontiguousarray(x_bits[order]), np.ascontiguousarray(y[order])
+    if x_bits.shape[0] < y.size or y.shape[0] < y.size:
+        raise IndexError("fewer rows than labels")
+    order = np.random.default_rng(seed).permutation(y.size).astype(np.uint32)
     losses = np.zeros(epochs, np.float32)
-    _lib.check(_lib.load().faco_mlp_train(params.ctypes.data, xs.ctypes.data, ys.ctypes.data, ys.size, epochs,
-                                          batch, lr, losses.ctypes.data))
+    _lib.check(_lib.load().faco_mlp_train_order(params.ctypes.data, x_bits.ctypes.data, y.ctypes.data,
+                                                order.ctypes.data, y.size, epochs, batch, lr, losses.ctypes.data))
     return params, losses
 
 

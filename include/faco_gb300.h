@@ -354,6 +354,10 @@ int faco_mlp_gradient(const float* params, const uint16_t* x, const float* y, ui
  * (shuffle the rows first); params updated in place; mean loss per epoch. */
 int faco_mlp_train(float* params, const uint16_t* x, const float* y, uint32_t count, uint32_t epochs,
                    uint32_t batch, float learning_rate, float* epoch_losses);
+/* The same over the rows in `order` ([count] row numbers below count), taken
+ * on the device: a shuffled training without a shuffled copy of the rows. */
+int faco_mlp_train_order(float* params, const uint16_t* x, const float* y, const uint32_t* order, uint32_t count,
+                         uint32_t epochs, uint32_t batch, float learning_rate, float* epoch_losses);
 /* During a stepwise evaluation: features (and labels: edge of the colony's
  * global-best tour) of every candidate entry of every colony, rows ordered
  * (colony, node, rank); `rows` receives the row count (pass NULL outputs to
