@@ -367,10 +367,11 @@ __device__ __forceinline__ bool on_segment(int lo, int hi, int q) { return q >= 
 // certainly above it; so one pass over the row decides, with the total and
 // those two prefixes.  False where the margin leaves it open (the one-step
 // path then decides).  Rows of a multiple of four candidates are read four
-// at a time (8 + 16 bytes), one group ahead of the sums.
+// at a time (8 + 16 bytes), one group ahead of the sums; the caller has read
+// the first one (x, p).
 __device__ __forceinline__ bool follow_takes(const AntSmem& s, const node_t* row, const float* prow, std::uint32_t n,
                                              std::uint32_t k, std::uint32_t sel, std::uint32_t rel, std::uint32_t t0,
-                                             bool identity, int lo, int hi, float uf) {
+                                             bool identity, int lo, int hi, float uf, uint2 x, float4 p) {
     float total = 0.0f, before = 0.0f, upto = -1.0f;
     bool any = false, earlier = false;
     // (adding zero for a closed candidate leaves the sum as it is)
@@ -388,8 +389,6 @@ __device__ __forceinline__ bool follow_takes(const AntSmem& s, const node_t* row
     if ((k & 3u) == 0) {
         const uint2* rows = reinterpret_cast<const uint2*>(row);
         const float4* weights = reinterpret_cast<const float4*>(prow);
-        uint2 x = __ldg(rows);
-        float4 p = __ldg(weights);
 #pragma unroll 1
         for (std::uint32_t g = 1; g <= k / 4; ++g) {
             const uint2 xg = x;
@@ -476,6 +475,15 @@ __device__ inline std::uint32_t follow_batch(const AntSmem& s, const int2* xy, c
             hi = a < b ? b : a;
         }
     }
+    // the first candidates of the lane's row, before what decides whether they are needed
+    const node_t* row = in.primary + (size_t)cur * k;
+    const float* prow = products + (size_t)cur * k;
+    uint2 x = {0, 0};
+    float4 p4 = {0.0f, 0.0f, 0.0f, 0.0f};
+    if ((k & 3u) == 0) {
+        x = __ldg(reinterpret_cast<const uint2*>(row));
+        p4 = __ldg(reinterpret_cast<const float4*>(prow));
+    }
     if (ok) {
         const std::uint32_t pn = __ldg(parent_nbr + cur);
         ok = (sel == (pn & 0xffffu) || sel == (pn >> 16)) && !test_bit(s.visited, sel);
@@ -487,16 +495,14 @@ __device__ inline std::uint32_t follow_batch(const AntSmem& s, const int2* xy, c
     v.p = (std::uint32_t)p;
     v.t = (std::uint32_t)t;
     v.dir = D;
+    std::uint32_t tpos = 0, target_after = n;
     if (ok && !identity) {
-        const std::uint32_t tpos = v.current_pos();
-        ok = v.read(s, tpos + 1 == n ? 0 : tpos + 1) != sel;
+        tpos = v.current_pos();
+        target_after = v.read(s, tpos + 1 == n ? 0 : tpos + 1);
+        ok = target_after != sel;
     }
     // the roulette of this lane's step: serial FP32 sums in candidate order
-    if (ok) {
-        const node_t* row = in.primary + (size_t)cur * k;
-        const float* prow = products + (size_t)cur * k;
-        ok = follow_takes(s, row, prow, n, k, sel, rel, t0, identity, lo, hi, uf);
-    }
+    if (ok) ok = follow_takes(s, row, prow, n, k, sel, rel, t0, identity, lo, hi, uf, x, p4);
     // the leading run of taken steps
     const unsigned okm = __ballot_sync(kFull, ok);
     std::uint32_t f, first_lane;
@@ -513,53 +519,44 @@ __device__ inline std::uint32_t follow_batch(const AntSmem& s, const int2* xy, c
     if (f == 0) return 0;
     const bool taken = lane >= first_lane && lane < first_lane + f;
     // identity lanes of the chosen half all agree on `identity`
+    const std::uint32_t last_lane = first_lane + f - 1;
     const bool ident = __shfl_sync(kFull, identity ? 1 : 0, first_lane) != 0;
-    long long d = 0;
-    std::uint32_t moved = 0;
-    if (taken && !ident) {
-        // six-edge delta of CpuTour::relocate for this lane's step, its
-        // positions and tour neighbours read through the run with m = mr
-        const std::uint32_t tpos = v.current_pos(), npos = v.source_pos(D);
-        std::uint32_t target_after = n, previous = n, after = n;
-#pragma unroll 1
-        for (int t = 0; t < 3; ++t) {   // one copy of the run's read in the code
-            const std::uint32_t at = t == 0 ? (tpos + 1 == n ? 0 : tpos + 1)
-                                   : t == 1 ? (npos == 0 ? n - 1 : npos - 1) : (npos + 1 == n ? 0 : npos + 1);
-            const std::uint32_t x = v.read(s, at);
-            if (t == 0) target_after = x;
-            else if (t == 1) previous = x;
-            else after = x;
-        }
-        // added (previous,after) (cur,sel) (sel,target_after), removed
-        // (previous,sel) (sel,after) (cur,target_after): one loop, so that
-        // the batch's code holds one copy of the distance
-#pragma unroll 1
-        for (int t = 0; t < 6; ++t) {
-            const std::uint32_t ea = t == 0 || t == 3 ? previous : t == 2 || t == 4 ? sel : cur;
-            const std::uint32_t eb = t == 0 || t == 4 ? after : t == 1 || t == 3 ? sel : target_after;
-            const int dd = euc2d(xy[ea], xy[eb]);
-            d += t < 3 ? dd : -dd;
-        }
-        moved = tpos < npos ? npos - tpos : tpos - npos + 1;
-    }
-    if (taken) atomicOr(&s.visited[sel >> 5], 1u << (sel & 31u));
-#pragma unroll
-    for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(kFull, d, o);
-    moved = __reduce_add_sync(kFull, moved);
-    current = __shfl_sync(kFull, sel, first_lane + f - 1);
-    cost += d;
-    r.steps += f;
+    const std::uint32_t last = __shfl_sync(kFull, sel, last_lane);
     if (!ident) {
-        const int Dt = __shfl_sync(kFull, D, first_lane);
-        const std::uint32_t pt = (std::uint32_t)__shfl_sync(kFull, p, first_lane);
-        const std::uint32_t tt = (std::uint32_t)__shfl_sync(kFull, t, first_lane);
+        // The six-edge deltas of CpuTour::relocate over the steps telescope:
+        // with s_1 .. s_f the nodes taken after c, T the node after c, X
+        // beside s_1 on the near side of the sources and Y beside s_f on the
+        // far side (each read through the run of its own step), they add up to
+        // (X,Y) + (c,s_1) + (s_f,T) - (X,s_1) - (s_f,Y) - (c,T): one length
+        // per lane instead of six in each.
+        const std::uint32_t npos = v.source_pos(D);
+        const std::uint32_t right = npos + 1 == n ? 0 : npos + 1, left = npos == 0 ? n - 1 : npos - 1;
+        std::uint32_t near_end = n, far_end = n, moved = 0;
+        if (taken) {
+            near_end = v.read(s, D > 0 ? left : right);
+            far_end = v.read(s, D > 0 ? right : left);
+            moved = tpos < npos ? npos - tpos : tpos - npos + 1;
+        }
+        const std::uint32_t X = __shfl_sync(kFull, near_end, first_lane), T = __shfl_sync(kFull, target_after, first_lane);
+        const std::uint32_t Y = __shfl_sync(kFull, far_end, last_lane), first = __shfl_sync(kFull, sel, first_lane);
+        int term = 0;
+        if (lane < 6) {
+            const std::uint32_t ea = lane == 0 || lane == 3 ? X : lane == 1 || lane == 5 ? current : last;
+            const std::uint32_t eb = lane == 0 || lane == 4 ? Y : lane == 1 || lane == 3 ? first : T;
+            const int dd = euc2d(xy[ea], xy[eb]);
+            term = lane < 3 ? dd : -dd;
+        }
+        cost += __reduce_add_sync(kFull, term);
+        r.moved += __reduce_add_sync(kFull, moved);
         r.nonidentity += f;
-        r.moved += moved;
-        run.p = pt;
-        run.t = tt;
-        run.dir = Dt;
+        run.p = (std::uint32_t)__shfl_sync(kFull, p, first_lane);
+        run.t = (std::uint32_t)__shfl_sync(kFull, t, first_lane);
+        run.dir = __shfl_sync(kFull, D, first_lane);
         run.m = m0 + f;
     }
+    if (taken) atomicOr(&s.visited[sel >> 5], 1u << (sel & 31u));
+    current = last;
+    r.steps += f;
     __syncwarp();
     return f;
 }
