@@ -648,9 +648,10 @@ void enqueue_update(faco_engine* e, cudaStream_t st, const std::uint32_t* list, 
         faco::fingerprint_kernel<<<(warps + 7) / 8, 256, 0, st>>>(e->colonies.get(), list, v.P.ants, colonies,
                                                                  v.P.zero_fingerprints);
     }
-    faco::colony_update_kernel<<<colonies, 256, 0, st>>>(e->d_instances.get(), e->colonies.get(), e->states.get(),
-                                                          v.P, v.trace_cap ? e->trace.get() : nullptr, list,
-                                                          v.count, v.trace_cap);
+    cuda_check(faco::launch_colony_update(e->d_instances.get(), e->colonies.get(), e->states.get(), v.P,
+                                          v.trace_cap ? e->trace.get() : nullptr, list, colonies, v.count,
+                                          v.trace_cap, st),
+               "colony update");
     if (v.P.trail_blocks > 1)
         faco::colony_trails_kernel<<<dim3(v.P.trail_blocks, colonies), 256, 0, st>>>(
             e->d_instances.get(), e->colonies.get(), e->states.get(), v.P, list);
@@ -734,6 +735,13 @@ void capture_graph(faco_engine* e, cudaStream_t st) {
 // inverse in global memory, coordinates read from global) lets large classes
 // run a full block per SM slot instead of one or two shared-memory-bound ants.
 constexpr std::uint32_t kGlobalWorkspaceFrom = 2048;   // auto: n_max above this may use it
+
+// A full panel's shared-memory blocks of that size hold an SM each, which a
+// class timed alone does not show but the other chains do: at N 5000-8166
+// (40 colonies x 64 ants) shared memory timed 0-11 % faster than the global
+// workspace in five panels, and the two panels that took it ran 120 instead of
+// 107 ms; at N 2300-2500 it timed 29 % faster and ran 51 instead of 67 ms.
+constexpr float kSharedHandicap = 1.15f;
 
 bool may_use_global(const faco_settings& c, std::uint32_t n_max) {
     return c.workspace == FACO_WORKSPACE_GLOBAL ||
@@ -838,6 +846,7 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
                         cuda_check(cudaEventElapsedTime(&one, t0, t1), "elapsed");
                         if (rep > 0) ms += one;   // first launch warms caches
                     }
+                    if (v.full && mode == faco::kModeEngine && may_use_global(c, cl.n_max)) ms *= kSharedHandicap;
                     if (best_ms == 0.0f || ms < best_ms) {
                         best_ms = ms;
                         cl.warps = w;

@@ -528,24 +528,46 @@ __device__ __forceinline__ float trail_value(float tau, std::uint32_t to, std::u
     return v;
 }
 
-__device__ __forceinline__ void trail_update(std::uint32_t n, std::uint32_t k, const node_t* primary,
-                                             const std::uint32_t* nbr, float ret, float tmin, float tmax, float inc,
-                                             const float* eta, float* trails, float* products, std::uint32_t first,
-                                             std::uint32_t stride) {
+__device__ __forceinline__ void trail_update(std::uint32_t n, std::uint32_t k, const node_t* __restrict__ primary,
+                                             const std::uint32_t* __restrict__ nbr, float ret, float tmin, float tmax,
+                                             float inc, const float* __restrict__ eta, float* __restrict__ trails,
+                                             float* __restrict__ products, std::uint32_t first, std::uint32_t stride) {
     const std::uint32_t cells = n * k;
     if ((k & 3u) == 0) {
-        for (std::uint32_t q = first; q * 4 < cells; q += stride) {
-            const std::uint32_t idx = q * 4, nb = nbr[idx / k];
-            const float4 t = *reinterpret_cast<const float4*>(trails + idx);
-            const float4 e = *reinterpret_cast<const float4*>(eta + idx);
-            const uint2 pr = *reinterpret_cast<const uint2*>(primary + idx);
-            float4 v;
-            v.x = trail_value(t.x, pr.x & 0xffffu, nb, ret, tmin, tmax, inc);
-            v.y = trail_value(t.y, pr.x >> 16, nb, ret, tmin, tmax, inc);
-            v.z = trail_value(t.z, pr.y & 0xffffu, nb, ret, tmin, tmax, inc);
-            v.w = trail_value(t.w, pr.y >> 16, nb, ret, tmin, tmax, inc);
-            *reinterpret_cast<float4*>(trails + idx) = v;
-            *reinterpret_cast<float4*>(products + idx) = make_float4(v.x * e.x, v.y * e.y, v.z * e.z, v.w * e.w);
+        // groups of four entries, two in flight; the group's row by carry
+        const std::uint32_t per_row = k / 4, groups = cells / 4, step_rows = stride / per_row,
+                            step_rest = stride - step_rows * per_row;
+        std::uint32_t row = first / per_row, rest = first - row * per_row;
+        for (std::uint32_t q = first; q < groups;) {
+            float4 t[2], e[2];
+            uint2 pr[2];
+            std::uint32_t nb[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const std::uint32_t at = q + u * stride;
+                if (at >= groups) continue;
+                t[u] = reinterpret_cast<const float4*>(trails)[at];
+                e[u] = reinterpret_cast<const float4*>(eta)[at];
+                pr[u] = reinterpret_cast<const uint2*>(primary)[at];
+                nb[u] = nbr[row];
+                row += step_rows;
+                rest += step_rest;
+                if (rest >= per_row) { rest -= per_row; ++row; }
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const std::uint32_t at = q + u * stride;
+                if (at >= groups) continue;
+                float4 v;
+                v.x = trail_value(t[u].x, pr[u].x & 0xffffu, nb[u], ret, tmin, tmax, inc);
+                v.y = trail_value(t[u].y, pr[u].x >> 16, nb[u], ret, tmin, tmax, inc);
+                v.z = trail_value(t[u].z, pr[u].y & 0xffffu, nb[u], ret, tmin, tmax, inc);
+                v.w = trail_value(t[u].w, pr[u].y >> 16, nb[u], ret, tmin, tmax, inc);
+                reinterpret_cast<float4*>(trails)[at] = v;
+                reinterpret_cast<float4*>(products)[at] = make_float4(v.x * e[u].x, v.y * e[u].y, v.z * e[u].z,
+                                                                      v.w * e[u].w);
+            }
+            q += 2 * stride;
         }
     } else {
         for (std::uint32_t idx = first; idx < cells; idx += stride) {
@@ -610,9 +632,11 @@ __device__ __forceinline__ std::uint32_t row_entropy_q(const float* tau, std::ui
     for (std::uint32_t j = 0; j < k; ++j) sum = sum + tau[j];
     if (!(sum > 0.0f)) return 0;
     float h = 0.0f;
-    for (std::uint32_t j = 0; j < k; ++j) {
+#pragma unroll 4
+    for (std::uint32_t j = 0; j < k; ++j) {   // the divisions of four entries overlap, the sum stays in order
         const float p = tau[j] / sum;
-        if (p > 0.0f) h = h - p * own_log2(p);
+        const float term = p * own_log2(p > 0.0f ? p : 1.0f);
+        h = p > 0.0f ? h - term : h;
     }
     float hn = h / log2k;
     hn = hn < 0.0f ? 0.0f : hn > 1.0f ? 1.0f : hn;
@@ -636,24 +660,55 @@ __device__ __forceinline__ float apply_operation(int op, float l, float r, float
     return fminf(8.0f, fmaxf(-8.0f, v));
 }
 
-// Postfix interpreter (cuda/gp_score.cuh:64-102); feature(i) supplies terminal i.
+// A program in shared memory: the interpreter's loop reads one word per
+// instruction, ahead of its use (opcode | operand << 8).
+struct StagedProgram {
+    std::uint32_t length;
+    std::uint16_t code[64];
+    float constants[63];
+};
+
+__device__ __forceinline__ void stage_program(const Program& p, StagedProgram& to, std::uint32_t lane) {
+    for (std::uint32_t i = lane; i < 63; i += 32) {
+        to.code[i] = (std::uint16_t)(p.opcode[i] | p.operand[i] << 8);
+        to.constants[i] = p.constants[i];
+    }
+    if (lane == 0) {
+        to.length = p.length;
+        to.code[63] = 0;
+    }
+}
+
+// Postfix interpreter (cuda/gp_score.cuh:64-102); feature(i) supplies terminal
+// i.  The top of the stack stays in a register; the rest is one shared column
+// per lane (stack[d][lane], 15 deep).  A chain of one latency after the other:
+// from global memory with the stack in local memory a 63-node program took
+// 11-14 thousand cycles.
 template <class Feature>
-__device__ __forceinline__ float eval_program(const Program& p, Feature feature) {
-    float stack[16];
-    int top = 0;
-    for (int i = 0; i < p.length; ++i) {
-        const int op = p.opcode[i];
-        if (op == 0) stack[top++] = feature(p.operand[i]);
-        else if (op == 1) stack[top++] = p.constants[p.operand[i]];
-        else {
-            const int arity = op == 7 ? 1 : op == 10 ? 3 : 2;
-            const float t = arity == 3 ? stack[--top] : 0.0f;
-            const float r = arity >= 2 ? stack[--top] : 0.0f;
-            const float l = stack[--top];
-            stack[top++] = apply_operation(op, l, r, t);
+__device__ __forceinline__ float eval_program(const StagedProgram& p, float (*stack)[32], std::uint32_t lane,
+                                              Feature feature) {
+    float top = 0.0f;
+    int depth = 0;                 // entries below `top`, which is the first push's when depth < 0
+    --depth;
+    std::uint32_t next = p.code[0];
+#pragma unroll 1
+    for (std::uint32_t i = 0; i < p.length; ++i) {
+        const std::uint32_t op = next & 255u, operand = next >> 8;
+        next = p.code[i + 1];
+        if (op < 2) {
+            if (depth >= 0) stack[depth][lane] = top;
+            ++depth;
+            top = op == 0 ? feature((int)operand) : p.constants[operand];
+        } else if (op == 7) {
+            top = apply_operation(7, top, 0.0f, 0.0f);
+        } else {
+            const float t = op == 10 ? top : 0.0f;
+            const float r = op == 10 ? stack[--depth][lane] : top;
+            const float l = stack[--depth][lane];
+            top = apply_operation((int)op, l, r, t);
         }
     }
-    return stack[0];
+    return top;
 }
 
 // First maximum within 1e-6 among legal lanes (score_cpu rule); 32 if none.
@@ -672,16 +727,16 @@ __device__ __forceinline__ std::uint32_t choose_action(float value, bool legal, 
 // stride-wide window is; the first maximum within 1e-6 wins.  Role scores
 // go to slots 0-1, 2-5 and 6-9 of `role_scores` (may be null).
 template <class FeatureOf>
-__device__ __forceinline__ std::uint32_t choose_conditional(const Program* trees, FeatureOf feature_of,
-                                                            std::uint32_t mask, std::uint32_t lane,
-                                                            float* role_scores) {
+__device__ __forceinline__ std::uint32_t choose_conditional(const StagedProgram* trees, float (*stack)[32],
+                                                            FeatureOf feature_of, std::uint32_t mask,
+                                                            std::uint32_t lane, float* role_scores) {
     std::uint32_t prefix = 0;
 #pragma unroll 1
     for (int role = 0; role < 3; ++role) {
         const std::uint32_t width = role == 0 ? 2u : 4u, stride = role == 0 ? 16u : role == 1 ? 4u : 1u;
         const std::uint32_t action = prefix + (lane < width ? lane : 0u) * stride;
         const bool legal = lane < width && ((mask >> action) & ((1u << stride) - 1u)) != 0u;
-        const float value = eval_program(trees[role], [&](int i) { return feature_of(i, action); });
+        const float value = eval_program(trees[role], stack, lane, [&](int i) { return feature_of(i, action); });
         if (role_scores && lane < width) role_scores[(role == 0 ? 0 : role == 1 ? 2 : 6) + lane] = value;
         const std::uint32_t pick = choose_action(value, legal, lane);
         prefix += stride * (pick < 32u ? pick : 0u);
@@ -805,17 +860,34 @@ __device__ __forceinline__ long long band_limit(long long global_cost) {
     return (long long)floor((double)global_cost * (1 + kArchiveBand));
 }
 
+// The least candidate of the warp by (cost, fingerprint, index), in every
+// lane; lanes without one hold (LLONG_MAX, all ones, 0xffffffff).
+__device__ __forceinline__ void warp_least(std::uint32_t& best, long long& cost, Fingerprint& id) {
+#pragma unroll 1
+    for (int o = 16; o; o >>= 1) {
+        const std::uint32_t ob = __shfl_xor_sync(kFull, best, o);
+        const long long oc = __shfl_xor_sync(kFull, cost, o);
+        const Fingerprint oi{__shfl_xor_sync(kFull, id.first, o), __shfl_xor_sync(kFull, id.second, o)};
+        const bool less = (oi.first < id.first) | ((oi.first == id.first) & (oi.second < id.second));
+        const bool same = (oi.first == id.first) & (oi.second == id.second);
+        const bool take = (oc < cost) | ((oc == cost) & (less | (same & (ob < best))));
+        best = take ? ob : best;
+        cost = take ? oc : cost;
+        id.first = take ? oi.first : id.first;
+        id.second = take ? oi.second : id.second;
+    }
+}
+
 // Archive selection by warp 0 (update_control's slot loop): the global best
 // first, then up to 3 distinct tours of the old archive and the batch within
 // 2 % of the global cost, each the least by (cost, fingerprint, canonical
 // order, candidate index).
 __device__ std::uint32_t ref_archive_select(const CandidateView& v, const ColonyState& st, std::uint32_t A,
-                                            bool improved, std::uint32_t n, std::uint32_t lane,
+                                            bool improved, std::uint32_t n, std::uint32_t lane, long long limit,
                                             std::uint32_t* excluded, std::uint32_t* chosen) {
     const std::uint32_t total = kArchive + A;
     for (std::uint32_t w = lane; w < (total + 31) / 32; w += 32) excluded[w] = 0;
     __syncwarp();
-    const long long limit = band_limit(st.global_cost);
     auto is_excluded = [&](std::uint32_t c) { return (excluded[c >> 5] >> (c & 31u)) & 1u; };
     auto eligible = [&](std::uint32_t c) {
         if (c < kArchive && c >= v.ctl.archive_size) return false;
@@ -845,25 +917,19 @@ __device__ std::uint32_t ref_archive_select(const CandidateView& v, const Colony
         __syncwarp();
     };
     add(improved ? kArchive + st.iteration_best : 0u);
+#pragma unroll 1
     for (std::uint32_t slot = 1; slot < kArchive; ++slot) {
         std::uint32_t best = 0xffffffffu;
-        long long bc = 0;
-        Fingerprint bi{0, 0};
+        long long bc = LLONG_MAX;
+        Fingerprint bi{~0ull, ~0ull};
+#pragma unroll 1
         for (std::uint32_t c = lane; c < total; c += 32) {
             if (!eligible(c)) continue;
             const long long cc = v.cost(c);
             const Fingerprint ci = v.id(c);
             if (best == 0xffffffffu || cc < bc || (cc == bc && fp_less(ci, bi))) { best = c; bc = cc; bi = ci; }
         }
-        for (int o = 16; o; o >>= 1) {
-            const std::uint32_t ob = __shfl_xor_sync(kFull, best, o);
-            const long long oc = __shfl_xor_sync(kFull, bc, o);
-            const Fingerprint oi{__shfl_xor_sync(kFull, bi.first, o), __shfl_xor_sync(kFull, bi.second, o)};
-            const bool take = ob != 0xffffffffu &&
-                              (best == 0xffffffffu || oc < bc ||
-                               (oc == bc && (fp_less(oi, bi) || (fp_equal(oi, bi) && ob < best))));
-            if (take) { best = ob; bc = oc; bi = oi; }
-        }
+        warp_least(best, bc, bi);
         if (best == 0xffffffffu) break;
         // equal cost and fingerprint with another tour: canonical order decides
         for (std::uint32_t base = 0; base < total; base += 32) {
@@ -886,12 +952,12 @@ __device__ std::uint32_t ref_archive_select(const CandidateView& v, const Colony
 // fingerprint): a group of identical tours acts as its first member, and the
 // least by (cost, fingerprint, index) needs no tour comparison.
 __device__ std::uint32_t ref_archive_select_groups(const CandidateView& v, const ColonyState& st, std::uint32_t A,
-                                                   bool improved, std::uint32_t lane, const std::uint16_t* rep,
-                                                   std::uint32_t* excluded, std::uint32_t* chosen) {
+                                                   bool improved, std::uint32_t lane, long long limit,
+                                                   const std::uint16_t* rep, std::uint32_t* excluded,
+                                                   std::uint32_t* chosen) {
     const std::uint32_t total = kArchive + A;
     for (std::uint32_t w = lane; w < (total + 31) / 32; w += 32) excluded[w] = 0;
     __syncwarp();
-    const long long limit = band_limit(st.global_cost);
     const std::uint32_t first = improved ? kArchive + st.iteration_best : 0u;
     if (lane == 0) {
         chosen[0] = first;
@@ -899,26 +965,23 @@ __device__ std::uint32_t ref_archive_select_groups(const CandidateView& v, const
     }
     __syncwarp();
     std::uint32_t count = 1;
+#pragma unroll 1
     for (std::uint32_t slot = 1; slot < kArchive; ++slot) {
         std::uint32_t best = 0xffffffffu;
-        long long bc = 0;
-        Fingerprint bi{0, 0};
+        long long bc = LLONG_MAX;
+        Fingerprint bi{~0ull, ~0ull};
+#pragma unroll 1
         for (std::uint32_t c = lane; c < total; c += 32) {
             if (rep[c] != c || ((excluded[c >> 5] >> (c & 31u)) & 1u)) continue;
-            const long long cc = v.cost(c);
+            // (volatile keeps the loop's loads in the loop: moved out of it
+            // and over the slots they took 33 thousand cycles instead of 8)
+            const long long cc = c < kArchive ? v.ctl.archive_cost[c]
+                                              : static_cast<const volatile long long*>(v.costs)[c - kArchive];
             if (cc > limit) continue;
             const Fingerprint ci = v.id(c);
             if (best == 0xffffffffu || cc < bc || (cc == bc && fp_less(ci, bi))) { best = c; bc = cc; bi = ci; }
         }
-        for (int o = 16; o; o >>= 1) {
-            const std::uint32_t ob = __shfl_xor_sync(kFull, best, o);
-            const long long oc = __shfl_xor_sync(kFull, bc, o);
-            const Fingerprint oi{__shfl_xor_sync(kFull, bi.first, o), __shfl_xor_sync(kFull, bi.second, o)};
-            const bool take = ob != 0xffffffffu &&
-                              (best == 0xffffffffu || oc < bc ||
-                               (oc == bc && (fp_less(oi, bi) || (fp_equal(oi, bi) && ob < best))));
-            if (take) { best = ob; bc = oc; bi = oi; }
-        }
+        warp_least(best, bc, bi);
         if (best == 0xffffffffu) break;
         if (lane == 0) {
             chosen[count] = best;
@@ -945,7 +1008,10 @@ struct RefShared {
     long long chosen_cost[kArchive];
     Fingerprint chosen_id[kArchive];
     std::uint32_t count, alternative, mask, action, largest;
+    StagedProgram trees[3];
+    float stack[15][32];
     float gap[2], difference, elapsed, stagnation;
+    long long limit;                      // archive band of the global best
 };
 
 __device__ __forceinline__ CandidateView candidates(const ColonyView& cv, const RefShared& sh, std::uint32_t A) {
@@ -970,6 +1036,7 @@ __device__ void ref_update(const ColonyView& cv, const InstanceView& in, const C
             sh.ant_p0[a] = cv.ant_p0[a];
         }
     if (threadIdx.x == 0) sh.collision = 0;
+    if (threadIdx.x == 64) sh.limit = band_limit(st.global_cost);
     __syncthreads();
     const bool improved = st.global_cost < ctl.tracked_global;
     const CandidateView v = candidates(cv, sh, A);
@@ -982,6 +1049,7 @@ __device__ void ref_update(const ColonyView& cv, const InstanceView& in, const C
             r = (std::uint16_t)c;
             const Fingerprint fc = v.id(c);
             const long long cc = v.cost(c);
+#pragma unroll 1
             for (std::uint32_t q = 0; q < c; ++q) {
                 if (q < kArchive && q >= ctl.archive_size) continue;
                 if (!fp_equal(v.id(q), fc)) continue;
@@ -1000,10 +1068,11 @@ __device__ void ref_update(const ColonyView& cv, const InstanceView& in, const C
     __syncthreads();
     if (warp == 0) {
         const std::uint32_t count =
-            sh.collision ? ref_archive_select(v, st, A, improved, n, lane, sh.excluded, sh.chosen)
-                         : ref_archive_select_groups(v, st, A, improved, lane, sh.rep, sh.excluded, sh.chosen);
+            sh.collision ? ref_archive_select(v, st, A, improved, n, lane, sh.limit, sh.excluded, sh.chosen)
+                         : ref_archive_select_groups(v, st, A, improved, lane, sh.limit, sh.rep, sh.excluded, sh.chosen);
         if (lane == 0) {
             sh.count = count;
+#pragma unroll 1
             for (std::uint32_t i = 0; i < count; ++i) {
                 sh.chosen_cost[i] = v.cost(sh.chosen[i]);
                 sh.chosen_id[i] = v.id(sh.chosen[i]);
@@ -1023,6 +1092,7 @@ __device__ void ref_update(const ColonyView& cv, const InstanceView& in, const C
                 if (P.ls_limit) wa = (double)cv.ant_counts[3 * a + 1] / (double)P.ls_limit;
             }
             returned += __popc(__ballot_sync(kFull, back));
+#pragma unroll 1
             for (std::uint32_t j = 0; j < 32 && base + j < A; ++j) work += __shfl_sync(kFull, wa, j);
         }
         if (lane == 0) {
@@ -1040,18 +1110,29 @@ __device__ void ref_update(const ColonyView& cv, const InstanceView& in, const C
         }
     }
     __syncthreads();
-    // chosen tours into the other half of the archive buffer
-    const std::uint32_t next = ctl.side ^ 1u, count = sh.count;
-    for (std::uint32_t i = threadIdx.x; i < count * n; i += blockDim.x) {
-        const std::uint32_t slot = i / n, p = i % n;
-        const node_t node = v.ref(sh.chosen[slot]).tour[p];
+    // chosen tours into the other half of the archive buffer: the slots side
+    // by side, eight nodes per thread (tour rows are 16-byte aligned, n_pad nodes)
+    const std::uint32_t next = ctl.side ^ 1u, count = sh.count, share = blockDim.x / kArchive;
+    const std::uint32_t slot = threadIdx.x / share;
+    if (slot < count) {
+        const node_t* tour = v.ref(sh.chosen[slot]).tour;
         node_t* dst = archive_tour(cv, next, slot);
-        dst[p] = node;
-        dst[cv.n_pad + node] = (node_t)p;
-        if (node == 0) sh.next_p0[slot] = p;
+        for (std::uint32_t g = threadIdx.x - slot * share; g * 8 < n; g += share) {
+            const uint4 x = reinterpret_cast<const uint4*>(tour)[g];
+            reinterpret_cast<uint4*>(dst)[g] = x;
+            const std::uint32_t words[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const std::uint32_t at = g * 8 + u, node = (words[u >> 1] >> (16 * (u & 1))) & 0xffffu;
+                if (at >= n) continue;
+                dst[cv.n_pad + node] = (node_t)at;
+                if (node == 0) sh.next_p0[slot] = at;
+            }
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
+#pragma unroll 1
         for (std::uint32_t i = 0; i < kArchive; ++i) {
             ctl.archive_cost[i] = i < count ? sh.chosen_cost[i] : 0;
             ctl.archive_id[i] = i < count ? sh.chosen_id[i] : Fingerprint{0, 0};
@@ -1072,6 +1153,8 @@ __device__ void ref_decide(const ColonyView& cv, const InstanceView& in, ColonyS
     const std::uint32_t n = in.n, k = in.k;
     const std::uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const std::uint32_t side = ctl.side, size = ctl.archive_size;
+    if (warp >= 2 && warp < 5 && (warp == 2 || cv.controller_kind == 1))
+        stage_program(cv.program[warp - 2], sh.trees[warp - 2], lane);
     if (warp == 0) {
         // alternative reference: the archive tour other than the active one
         // that differs most from it on the sampled nodes (control_cpu.cpp:46-63);
@@ -1103,10 +1186,12 @@ __device__ void ref_decide(const ColonyView& cv, const InstanceView& in, ColonyS
                 missing[i] += (cs != ps[h] && cs != pp[h]) + (cp != ps[h] && cp != pp[h]);
             }
         }
+#pragma unroll 1
+        for (int o = 16; o; o >>= 1)
 #pragma unroll
-        for (std::uint32_t i = 0; i < kArchive; ++i)
-            for (int o = 16; o; o >>= 1) missing[i] += __shfl_xor_sync(kFull, missing[i], o);
+            for (std::uint32_t i = 0; i < kArchive; ++i) missing[i] += __shfl_xor_sync(kFull, missing[i], o);
         std::uint32_t alt = kArchive, largest = 0;
+#pragma unroll 1
         for (std::uint32_t i = 0; i < size; ++i) {
             const TourRef ri{archive_tour(cv, side, i), archive_tour(cv, side, i) + cv.n_pad, ctl.archive_p0[i]};
             if (fp_equal(ctl.archive_id[i], ctl.active_id) && warp_canonical_compare(ri, parent, n, lane) == 0)
@@ -1125,17 +1210,19 @@ __device__ void ref_decide(const ColonyView& cv, const InstanceView& in, ColonyS
         if (lane == 0) {
             sh.alternative = alt;
             sh.largest = largest;
-            sh.gap[0] = (float)unit_clip(((double)st.parent_cost / (double)st.global_cost - 1) / kArchiveBand);
             sh.gap[1] = alt < kArchive ? (float)unit_clip(((double)ctl.archive_cost[alt] / (double)st.global_cost - 1) /
                                                           kArchiveBand)
                                        : 0.0f;
             sh.difference = alt < kArchive ? (float)largest / (float)(2 * in.sample_count) : 0.0f;
             sh.mask = cv.action_mask & (alt < kArchive ? 0xFFFFFFFFu : 0xFFFFu);
-            sh.elapsed = (float)unit_clip((double)((unsigned long long)batch * P.ants) /
-                                          (double)((unsigned long long)P.total_iterations * P.ants));
-            const unsigned long long stag = ctl.stagnant_batches;
-            sh.stagnation = (float)(stag < 32 ? (double)stag / 32.0 : 1.0);
         }
+    } else if (threadIdx.x == 32) {
+        // what does not depend on the alternative, in a warp of its own (FP64 divisions)
+        sh.gap[0] = (float)unit_clip(((double)st.parent_cost / (double)st.global_cost - 1) / kArchiveBand);
+        sh.elapsed = (float)unit_clip((double)((unsigned long long)batch * P.ants) /
+                                      (double)((unsigned long long)P.total_iterations * P.ants));
+        const unsigned long long stag = ctl.stagnant_batches;
+        sh.stagnation = (float)(stag < 32 ? (double)stag / 32.0 : 1.0);
     }
     __syncthreads();
     const std::uint32_t alt = sh.alternative, count = n < kRegionNodes ? n : kRegionNodes;
@@ -1175,6 +1262,7 @@ __device__ void ref_decide(const ColonyView& cv, const InstanceView& in, ColonyS
                 const int2 a = in.xy[xn], b = in.xy[y];
                 half = 0.5 * (double)euc2d(a, b);
                 float tau = st.default_trail;
+#pragma unroll 1
                 for (std::uint32_t t = 0; t < k; ++t)
                     if (in.primary[(size_t)xn * k + t] == y) { tau = cv.trails[(size_t)xn * k + t]; break; }
 #pragma unroll
@@ -1195,11 +1283,13 @@ __device__ void ref_decide(const ColonyView& cv, const InstanceView& in, ColonyS
                 ex = unit_clip(((half + other) / scale - 1) / 3);
             }
             double excess = 0, strength = 0;
+#pragma unroll 1
             for (std::uint32_t q = 0; q < count; ++q) {
                 excess += __shfl_sync(kFull, ex, 2 * q);
                 strength += __shfl_sync(kFull, strength_v, 2 * q);
                 strength += __shfl_sync(kFull, strength_v, 2 * q + 1);
             }
+#pragma unroll 1
             for (int o = 16; o; o >>= 1) {
                 dis += __shfl_xor_sync(kFull, dis, o);
                 disp += __shfl_xor_sync(kFull, disp, o);
@@ -1236,10 +1326,10 @@ __device__ void ref_decide(const ColonyView& cv, const InstanceView& in, ColonyS
         if (cv.controller_kind == 1) {
             sh.scores[lane] = 0.0f;
             __syncwarp();
-            a = choose_conditional(cv.program, [&](int i, std::uint32_t act) { return sh.feat[i][act]; }, mask, lane,
-                                   sh.scores);
+            a = choose_conditional(sh.trees, sh.stack, [&](int i, std::uint32_t act) { return sh.feat[i][act]; }, mask,
+                                   lane, sh.scores);
         } else {
-            const float value = eval_program(*cv.program, [&](int i) { return sh.feat[i][lane]; });
+            const float value = eval_program(sh.trees[0], sh.stack, lane, [&](int i) { return sh.feat[i][lane]; });
             sh.scores[lane] = value;
             a = choose_action(value, (mask >> lane) & 1u, lane);
         }
@@ -1419,24 +1509,40 @@ __device__ __forceinline__ void write_trace(TraceRow& row, const ColonyState& st
 // evaluations) the controller decision for the next iteration.  Block b
 // updates colony list[b] (colony b when `list` is null); `colony_count` is
 // the evaluation's colony count.
-__global__ void __launch_bounds__(256) colony_update_kernel(const InstanceView* instances,
-                                                            const ColonyView* colonies, ColonyState* states,
-                                                            ColonyParams P, TraceRow* trace,
-                                                            const std::uint32_t* list,
-                                                            std::uint32_t colony_count, std::uint32_t trace_cap) {
+//
+// CONTROL 0: plain FACO, 1: the engine's own controllers (feature spec 3), 2:
+// the reference's (spec 2).  A kernel each: the spec-2 decision takes 128
+// registers, with which the block of a plain colony, 256 threads then, waited
+// for half an SM to fall idle.  An update is the serial link between a
+// colony's iterations and bound by latency: one read of the best tour writes
+// the parent, its neighbours and the incumbents, the two FP64 chains (trail
+// limits; parent source and deposit) run in two warps, and 512 threads hold
+// two groups of trail entries each.  One GB300, in thousand cycles of one
+// colony's update, before -> after: N=1000-2000 (trails apart) 15.6 -> 12.2,
+// spec 3 at N=500 52 -> 37, spec 2 at N=500 146 -> 88; whole runs: 128 x 32
+// ants at N=1000-2000 146.2 -> 141.8 ms, the uneven batch 84.2 -> 82.2.
+__host__ __device__ constexpr std::uint32_t update_threads(int control) { return control == 2 ? 256u : 512u; }
+
+template <int CONTROL>
+__global__ void __launch_bounds__(update_threads(CONTROL), CONTROL == 2 ? 2 : 3)
+colony_update_kernel(const InstanceView* instances, const ColonyView* colonies, ColonyState* states, ColonyParams P,
+                     TraceRow* trace, const std::uint32_t* list, std::uint32_t colony_count, std::uint32_t trace_cap) {
+    constexpr std::uint32_t kWarps = update_threads(CONTROL) / 32;
     const std::uint32_t c = list ? list[blockIdx.x] : blockIdx.x;
     const ColonyView cv = colonies[c];
     const InstanceView in = instances[cv.instance];
     const std::uint32_t n = in.n, k = in.k, A = P.ants;
-    const std::uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    __shared__ unsigned long long s_red[6][8];
+    const std::uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ unsigned long long s_red[6][kWarps];
     __shared__ ColonyState s_st;
-    __shared__ std::uint32_t s_best, s_improve_epoch, s_improve_global, s_from_epoch, s_restart;
+    __shared__ std::uint32_t s_from_epoch, s_restart;
     __shared__ float s_tmin, s_tmax, s_inc, s_feat[7];
-    __shared__ long long s_sum_final, s_sum_cons, s_best_cost;
+    __shared__ long long s_sum_final, s_sum_cons;
     __shared__ unsigned long long s_steps, s_evals;
     __shared__ std::uint32_t s_used_mne, s_parent_p0;
 
+    for (std::uint32_t w = threadIdx.x; w < sizeof(ColonyState) / 4; w += blockDim.x)
+        reinterpret_cast<std::uint32_t*>(&s_st)[w] = reinterpret_cast<const std::uint32_t*>(states + c)[w];
     // iteration best: first strict minimum over ants (costs are >= 0); work counters
     unsigned long long best = ~0ull, steps = 0, evals = 0, moved = 0, sum_final = 0, sum_cons = 0;
     for (std::uint32_t a = threadIdx.x; a < A; a += blockDim.x) {
@@ -1448,66 +1554,91 @@ __global__ void __launch_bounds__(256) colony_update_kernel(const InstanceView* 
         sum_final += (unsigned long long)cv.ant_costs[a];
         sum_cons += (unsigned long long)cv.ant_ccosts[a];
     }
-    for (int o = 16; o; o >>= 1) {
-        const unsigned long long other = __shfl_xor_sync(kFull, best, o);
-        best = other < best ? other : best;
-        steps += __shfl_xor_sync(kFull, steps, o);
-        evals += __shfl_xor_sync(kFull, evals, o);
-        moved += __shfl_xor_sync(kFull, moved, o);
-        sum_final += __shfl_xor_sync(kFull, sum_final, o);
-        sum_cons += __shfl_xor_sync(kFull, sum_cons, o);
-    }
-    if (lane == 0) {
-        s_red[0][warp] = best; s_red[1][warp] = steps; s_red[2][warp] = evals;
-        s_red[3][warp] = moved; s_red[4][warp] = sum_final; s_red[5][warp] = sum_cons;
+    const std::uint32_t used = A < 32 * kWarps ? (A + 31) / 32 : kWarps;   // warps that hold ants
+    if (warp < used) {
+        for (int o = 16; o; o >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(kFull, best, o);
+            best = other < best ? other : best;
+            steps += __shfl_xor_sync(kFull, steps, o);
+            evals += __shfl_xor_sync(kFull, evals, o);
+            moved += __shfl_xor_sync(kFull, moved, o);
+            sum_final += __shfl_xor_sync(kFull, sum_final, o);
+            sum_cons += __shfl_xor_sync(kFull, sum_cons, o);
+        }
+        if (lane == 0) {
+            s_red[0][warp] = best; s_red[1][warp] = steps; s_red[2][warp] = evals;
+            s_red[3][warp] = moved; s_red[4][warp] = sum_final; s_red[5][warp] = sum_cons;
+        }
     }
     __syncthreads();
+    best = s_red[0][0];
+    for (std::uint32_t w = 1; w < used; ++w) best = s_red[0][w] < best ? s_red[0][w] : best;
+    const std::uint32_t ib = (std::uint32_t)(best & 0xffffu);
+    const long long cost = (long long)(best >> 16);
+    const bool ie = cost < s_st.epoch_cost, ig = cost < s_st.global_cost;
+    const long long epoch_cost = ie ? cost : s_st.epoch_cost;
     if (threadIdx.x == 0) {
-        for (std::uint32_t w = 1; w < warps; ++w) {
-            best = s_red[0][w] < best ? s_red[0][w] : best;
+        float tmin, tmax;
+        trail_limits(epoch_cost, P.retention, P.p_root, k, tmin, tmax);
+        s_tmin = tmin;
+        s_tmax = tmax;
+    }
+    if (threadIdx.x == 32) {
+        const bool from_epoch = source_uniform(cv.key, s_st.iteration) < P.epoch_source_probability;
+        s_from_epoch = from_epoch;
+        s_inc = (float)(1.0 / (double)(from_epoch ? epoch_cost : cost));
+    }
+    const std::uint32_t vectors = (n + 7) / 8;   // 8 nodes; rows are padded to whole ones
+    const node_t* best_tour = cv.ant_tours + (size_t)ib * cv.n_pad;
+    for (std::uint32_t g = threadIdx.x; (ie || ig) && g < vectors; g += blockDim.x) {
+        const uint4 x = reinterpret_cast<const uint4*>(best_tour)[g];
+        if (ie) reinterpret_cast<uint4*>(cv.epoch)[g] = x;
+        if (ig) reinterpret_cast<uint4*>(cv.global)[g] = x;
+    }
+    __syncthreads();
+    // the parent (the epoch's best, which may be this iteration's) and its packed neighbours
+    const bool fe = s_from_epoch;
+    const node_t* source = fe && !ie ? cv.epoch : best_tour;
+    for (std::uint32_t g = threadIdx.x; g < vectors; g += blockDim.x) {
+        const uint4 x = reinterpret_cast<const uint4*>(source)[g];
+        std::uint32_t before = source[g == 0 ? n - 1 : 8 * g - 1];
+        const std::uint32_t after = source[8 * g + 8 < n ? 8 * g + 8 : 0];
+        reinterpret_cast<uint4*>(cv.parent)[g] = x;
+        const std::uint32_t words[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (std::uint32_t u = 0; u < 8; ++u) {
+            const std::uint32_t i = 8 * g + u, node = (words[u >> 1] >> (16 * (u & 1))) & 0xffffu;
+            if (i >= n) continue;
+            const std::uint32_t next = i + 1 == n || u == 7 ? after : (words[(u + 1) >> 1 & 3] >> (16 * ((u + 1) & 1))) & 0xffffu;
+            cv.parent_nbr[node] = next | before << 16;
+            before = node;
+            if (CONTROL == 2 && node == 0) s_parent_p0 = i;
+        }
+    }
+    if (threadIdx.x == 0) {
+        for (std::uint32_t w = 0; w < used; ++w) {
+            if (w == 0) steps = evals = moved = sum_final = sum_cons = 0;
             steps += s_red[1][w]; evals += s_red[2][w]; moved += s_red[3][w];
             sum_final += s_red[4][w]; sum_cons += s_red[5][w];
         }
-        ColonyState st = states[c];
-        const std::uint32_t ib = (std::uint32_t)(best & 0xffffu);
-        const long long cost = (long long)(best >> 16);
-        const bool ie = cost < st.epoch_cost, ig = cost < st.global_cost;
-        if (ie) st.epoch_cost = cost;
+        ColonyState& st = s_st;
+        st.epoch_cost = epoch_cost;
         if (ig) { st.global_cost = cost; st.last_improvement = st.iteration + 1; }
-        trail_limits(st.epoch_cost, P.retention, P.p_root, k, st.tau_min, st.tau_max);
-        const bool from_epoch = source_uniform(cv.key, st.iteration) < P.epoch_source_probability;
-        st.parent_cost = from_epoch ? st.epoch_cost : cost;
+        st.tau_min = s_tmin;
+        st.tau_max = s_tmax;
+        st.parent_cost = fe ? epoch_cost : cost;
         st.iteration_best = ib;
         st.iteration_best_cost = cost;
-        st.source_is_epoch = from_epoch;
+        st.source_is_epoch = fe;
         st.construction_steps += steps;
         st.ls_evaluations += evals;
         st.reversed_elements += moved;
         *cv.walk = (std::uint32_t)(steps / A);
         st.default_trail = fmaxf(st.tau_min, st.default_trail * P.retention_f);
-        s_st = st;
-        s_best = ib; s_improve_epoch = ie; s_improve_global = ig; s_from_epoch = from_epoch;
-        s_tmin = st.tau_min; s_tmax = st.tau_max;
-        s_inc = (float)(1.0 / (double)st.parent_cost);
-        s_sum_final = (long long)sum_final; s_sum_cons = (long long)sum_cons; s_best_cost = cost;
+        s_sum_final = (long long)sum_final; s_sum_cons = (long long)sum_cons;
         s_steps = steps; s_evals = evals; s_used_mne = st.mne_target;
         s_restart = 0;
     }
-    __syncthreads();
-    const node_t* best_tour = cv.ant_tours + (size_t)s_best * cv.n_pad;
-    const bool ie = s_improve_epoch, ig = s_improve_global, fe = s_from_epoch;
-    for (std::uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const node_t v = best_tour[i];
-        if (ie) cv.epoch[i] = v;
-        if (ig) cv.global[i] = v;
-        const node_t p = fe ? cv.epoch[i] : v;
-        cv.parent[i] = p;
-        if (p == 0) s_parent_p0 = i;
-    }
-    __syncthreads();
-    for (std::uint32_t i = threadIdx.x; i < n; i += blockDim.x)
-        cv.parent_nbr[cv.parent[i]] = (std::uint32_t)cv.parent[i + 1 == n ? 0 : i + 1] |
-                                      ((std::uint32_t)cv.parent[i == 0 ? n - 1 : i - 1] << 16);
     __syncthreads();
     if (P.trail_blocks <= 1) {
         trail_update(n, k, in.primary, cv.parent_nbr, P.retention_f, s_tmin, s_tmax, s_inc, cv.eta, cv.trails,
@@ -1518,7 +1649,7 @@ __global__ void __launch_bounds__(256) colony_update_kernel(const InstanceView* 
         }
     }
     std::int32_t action = -1;
-    if (P.ref_control) {
+    if constexpr (CONTROL == 2) {
         // the 12-feature controller: the trace row holds the action this
         // batch ran with; archive and feedback; the next batch's decision
         __shared__ RefShared s_ref;
@@ -1533,8 +1664,18 @@ __global__ void __launch_bounds__(256) colony_update_kernel(const InstanceView* 
         if (s_st.iteration + 1 < P.total_iterations)
             ref_decide(cv, in, s_st, P, c, colony_count, s_st.iteration + 1, s_parent_p0, s_ref);
         if (threadIdx.x == 0) *cv.control = s_ref.ctl;
-    } else if (P.controlled && cv.program) {
+    } else if (CONTROL == 1 && cv.program) {
         // mean normalised entropy of the trail rows (exact integer sum)
+        __shared__ StagedProgram s_trees[3];
+        __shared__ float s_stack[15][32], s_action[3][32];
+        if (warp == 5) {
+            // the descriptors of action `lane`: MNE level, start region, restart flag
+            s_action[0][lane] = (float)(lane & 3u) / 3.0f;
+            s_action[1][lane] = (float)((lane >> 2) & 3u) / 3.0f;
+            s_action[2][lane] = lane >= 16u ? 1.0f : 0.0f;
+        }
+        if (warp >= 2 && warp < 5 && (warp == 2 || cv.controller_kind == 1))
+            stage_program(cv.program[warp - 2], s_trees[warp - 2], lane);
         __syncthreads();
         unsigned long long q = 0;
         for (std::uint32_t row = threadIdx.x; row < n; row += blockDim.x)
@@ -1542,32 +1683,35 @@ __global__ void __launch_bounds__(256) colony_update_kernel(const InstanceView* 
         for (int o = 16; o; o >>= 1) q += __shfl_xor_sync(kFull, q, o);
         if (lane == 0) s_red[0][warp] = q;
         __syncthreads();
-        if (threadIdx.x == 0) {
-            for (std::uint32_t w = 1; w < warps; ++w) q += s_red[0][w];
+        if (lane == 0 && warp < 7) {
+            // one feature per warp: their FP64 and FP32 divisions side by side
             const ColonyState& st = s_st;
             const std::uint32_t t1 = st.iteration + 1, stag = t1 - st.last_improvement, age = t1 - st.last_restart;
-            const long long b = s_best_cost;
-            s_feat[0] = (float)t1 / (float)P.total_iterations;
-            s_feat[1] = (float)stag / (float)(stag + 16);
-            s_feat[2] = clamp01((double)(s_sum_final - (long long)A * b) / ((double)A * (double)b));
-            s_feat[3] = clamp01((double)q * (1.0 / 1048576.0) / (double)n);
-            s_feat[4] = (float)st.restarts / (float)(st.restarts + 1);
-            s_feat[5] = clamp01((double)(s_sum_cons - s_sum_final) / (double)s_sum_cons * 10.0);
-            s_feat[6] = (float)age / (float)(age + 16);
+            const long long b = st.iteration_best_cost;
+            float f = 0.0f;
+            if (warp == 0) f = (float)t1 / (float)P.total_iterations;
+            else if (warp == 1) f = (float)stag / (float)(stag + 16);
+            else if (warp == 2) f = clamp01((double)(s_sum_final - (long long)A * b) / ((double)A * (double)b));
+            else if (warp == 3) {
+                q = 0;
+                for (std::uint32_t w = 0; w < kWarps; ++w) q += s_red[0][w];
+                f = clamp01((double)q * (1.0 / 1048576.0) / (double)n);
+            } else if (warp == 4) f = (float)st.restarts / (float)(st.restarts + 1);
+            else if (warp == 5) f = clamp01((double)(s_sum_cons - s_sum_final) / (double)s_sum_cons * 10.0);
+            else f = (float)age / (float)(age + 16);
+            s_feat[warp] = f;
         }
         __syncthreads();
         if (warp == 0) {
-            // features of action a: the 7 colony features, then its MNE level,
-            // start region and restart flag
+            // features of action a: the 7 colony features, then its descriptors
             auto feature_of = [&](int i, std::uint32_t a) {
-                return i < 7 ? s_feat[i] : i == 7 ? (float)(a & 3u) / 3.0f : i == 8 ? (float)((a >> 2) & 3u) / 3.0f
-                                                   : i == 9 ? (a >= 16u ? 1.0f : 0.0f) : 0.0f;
+                return i < 7 ? s_feat[i] : i < 10 ? s_action[i - 7][a] : 0.0f;
             };
             std::uint32_t a;
             if (cv.controller_kind == 1) {
-                a = choose_conditional(cv.program, feature_of, cv.action_mask, lane, nullptr);
+                a = choose_conditional(s_trees, s_stack, feature_of, cv.action_mask, lane, nullptr);
             } else {
-                const float value = eval_program(*cv.program, [&](int i) { return feature_of(i, lane); });
+                const float value = eval_program(s_trees[0], s_stack, lane, [&](int i) { return feature_of(i, lane); });
                 a = choose_action(value, (cv.action_mask >> lane) & 1u, lane);
             }
             if (lane == 0) {
@@ -1605,11 +1749,25 @@ __global__ void __launch_bounds__(256) colony_update_kernel(const InstanceView* 
     __syncthreads();
     if (threadIdx.x == 0) {
         ColonyState st = s_st;
-        if (trace && st.iteration < trace_cap && !P.ref_control)
+        if (trace && st.iteration < trace_cap && CONTROL != 2)
             write_trace(trace[(size_t)st.iteration * colony_count + c], st, s_used_mne, action, s_steps, s_evals);
         ++st.iteration;
         states[c] = st;
     }
+}
+
+cudaError_t launch_colony_update(const InstanceView* instances, const ColonyView* colonies, ColonyState* states,
+                                 const ColonyParams& P, TraceRow* trace, const std::uint32_t* list,
+                                 std::uint32_t blocks, std::uint32_t colony_count, std::uint32_t trace_cap,
+                                 cudaStream_t stream) {
+    const auto launch = [&](auto control) {
+        constexpr int kControl = decltype(control)::value;
+        colony_update_kernel<kControl><<<blocks, update_threads(kControl), 0, stream>>>(
+            instances, colonies, states, P, trace, list, colony_count, trace_cap);
+        return cudaGetLastError();
+    };
+    if (P.ref_control) return launch(std::integral_constant<int, 2>{});
+    return P.controlled ? launch(std::integral_constant<int, 1>{}) : launch(std::integral_constant<int, 0>{});
 }
 
 // The trail update of large candidate matrices, after the colony update has
@@ -1677,19 +1835,24 @@ __global__ void __launch_bounds__(kScoreWarps * 32)
 score_controllers_kernel(const Program* trees, const std::uint32_t* kinds, std::uint32_t replicas,
                          const float* features, const std::uint32_t* masks, float* scores, std::int32_t* actions,
                          std::uint32_t colonies, unsigned* error) {
-    __shared__ float staged[kScoreWarps][12][32];
+    __shared__ float staged[kScoreWarps][12][32], stacks[kScoreWarps][15][32];
+    __shared__ StagedProgram trees_of[kScoreWarps][3];
     const std::uint32_t colony = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (colony >= colonies) return;
     float(&mine)[12][32] = staged[threadIdx.x >> 5];
     stage_features(features, colony, colonies, lane, mine, error);
     const std::uint32_t controller = colony / replicas;
     const Program* slots = trees + 3 * (size_t)controller;
+    StagedProgram* own = trees_of[threadIdx.x >> 5];
+    float(*stack)[32] = stacks[threadIdx.x >> 5];
+    for (int t = 0; t < (kinds[controller] == 1 ? 3 : 1); ++t) stage_program(slots[t], own[t], lane);
+    __syncwarp();
     std::uint32_t chosen;
     if (kinds[controller] == 1) {
-        chosen = choose_conditional(slots, [&](int i, std::uint32_t a) { return mine[i][a]; }, masks[colony], lane,
+        chosen = choose_conditional(own, stack, [&](int i, std::uint32_t a) { return mine[i][a]; }, masks[colony], lane,
                                     scores + (size_t)colony * 32);
     } else {
-        const float value = eval_program(slots[0], [&](int i) { return mine[i][lane]; });
+        const float value = eval_program(own[0], stack, lane, [&](int i) { return mine[i][lane]; });
         scores[(size_t)colony * 32 + lane] = value;
         chosen = choose_action(value, (masks[colony] >> lane) & 1u, lane);
     }
@@ -1699,12 +1862,16 @@ score_controllers_kernel(const Program* trees, const std::uint32_t* kinds, std::
 __global__ void __launch_bounds__(kScoreWarps * 32)
 score_kernel(const Program* programs, std::uint32_t replicas, const float* features, const std::uint32_t* masks,
              float* scores, std::int32_t* actions, std::uint32_t colonies, unsigned* error) {
-    __shared__ float staged[kScoreWarps][12][32];
+    __shared__ float staged[kScoreWarps][12][32], stacks[kScoreWarps][15][32];
+    __shared__ StagedProgram program_of[kScoreWarps];
     const std::uint32_t colony = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (colony >= colonies) return;
     float(&mine)[12][32] = staged[threadIdx.x >> 5];
     stage_features(features, colony, colonies, lane, mine, error);
-    const float value = eval_program(programs[colony / replicas], [&](int i) { return mine[i][lane]; });
+    StagedProgram& own = program_of[threadIdx.x >> 5];
+    stage_program(programs[colony / replicas], own, lane);
+    __syncwarp();
+    const float value = eval_program(own, stacks[threadIdx.x >> 5], lane, [&](int i) { return mine[i][lane]; });
     scores[(size_t)colony * 32 + lane] = value;
     const std::uint32_t chosen = choose_action(value, (masks[colony] >> lane) & 1u, lane);
     if (lane == 0) actions[colony] = (std::int32_t)chosen;

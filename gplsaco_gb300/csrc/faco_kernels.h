@@ -65,10 +65,11 @@ __global__ void prior_rows_kernel(const InstanceView* instances, const ColonyVie
                                   const std::uint32_t* modes);
 __global__ void fingerprint_kernel(const ColonyView* colonies, const std::uint32_t* list, std::uint32_t ants,
                                    std::uint32_t colony_count, std::uint32_t zero);
-__global__ void colony_update_kernel(const InstanceView* instances, const ColonyView* colonies,
-                                     ColonyState* states, ColonyParams P, TraceRow* trace,
-                                     const std::uint32_t* list, std::uint32_t colony_count,
-                                     std::uint32_t trace_cap);
+// colony_update_kernel of `blocks` colonies (those of `list`, or all when null)
+cudaError_t launch_colony_update(const InstanceView* instances, const ColonyView* colonies, ColonyState* states,
+                                 const ColonyParams& P, TraceRow* trace, const std::uint32_t* list,
+                                 std::uint32_t blocks, std::uint32_t colony_count, std::uint32_t trace_cap,
+                                 cudaStream_t stream);
 __global__ void colony_trails_kernel(const InstanceView* instances, const ColonyView* colonies,
                                      const ColonyState* states, ColonyParams P, const std::uint32_t* list);
 __global__ void pheromone_step_kernel(std::uint32_t n, std::uint32_t k, const node_t* primary,
