@@ -59,6 +59,20 @@ __device__ __forceinline__ int euc2d(int2 p, int2 q) {
     return r;
 }
 
+// Programmatic dependent launch: lets the next kernel of the stream start its
+// prologue now; waits until the previous one is complete and its writes are
+// visible.  Both without effect in an ordinary launch.
+__device__ __forceinline__ void start_next_kernel() {
+#ifdef __CUDACC__
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+}
+__device__ __forceinline__ void wait_previous_kernel() {
+#ifdef __CUDACC__
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+#endif
+}
+
 // Philox4x32 with 10 rounds (Salmon, Moraes, Dror, Shaw, SC'11).
 struct uint4v { std::uint32_t x, y, z, w; };
 __device__ __forceinline__ uint4v philox4x32(std::uint32_t c0, std::uint32_t c1, std::uint32_t c2,

@@ -44,6 +44,13 @@ constexpr std::uint32_t kGraphIterations = 16;
 // workspace (2-opt) 1814 / 1857 at 54, 2195 / 1994 at 80.  Moving a line by a
 // fifth either way changes a run by less than 1 %.
 constexpr std::uint32_t kBatchFromOneWave = 30, kBatchFromFull = 48, kBatchFromGlobal = 60;
+// Up to this many ant warps per SM the iteration's kernels launch as
+// programmatic dependents: one N=100 colony (64 ants) 4.62 -> 4.46 ms, 32 x 32
+// ants with a prior 10.6 -> 9.9 ms.  Beyond, the waiting blocks keep other
+// chains' ants off the SMs: 32 x 128 ants at N=537 26.2 either way, the uneven
+// batch (27 warps per SM) 82.2 -> 85.3 ms, 256 x 32 ants at N=1000 111.8 ->
+// 118.4 ms.
+constexpr std::uint64_t kOverlapWarps = 8;
 // Automatic chain count: one chain per kColoniesPerChain colonies, at most kMaxChains.
 // Trail updates of more than 2 x kTrailCellsPerBlock entries per colony run in
 // colony_trails_kernel, one block per kTrailCellsPerBlock entries (at most
@@ -355,6 +362,7 @@ struct faco_engine {
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         bool full = false;                      // more ant warps than one wave of the GPU
+        bool overlap = false;                   // each kernel's prologue overlaps the kernel before it
         std::uint32_t batch_from = 0;           // AntLaunch::batch_from
     } eval;
     std::vector<cudaStream_t> branch_streams;
@@ -632,7 +640,7 @@ void enqueue_ants(faco_engine* e, cudaStream_t st) {
         const auto& c = v.classes[i];
         cudaStream_t bs = i == 0 ? st : e->branch_streams[i - 1];
         if (i > 0) cuda_check(cudaStreamWaitEvent(bs, e->branch_events[0], 0), "fork wait");
-        cuda_check(faco::launch_ant_kernel(c.mode, c.L, c.blocks, c.warps, c.smem, bs), "ant launch");
+        cuda_check(faco::launch_ant_kernel(c.mode, c.L, c.blocks, c.warps, c.smem, bs, v.overlap), "ant launch");
         if (i > 0) cuda_check(cudaEventRecord(e->branch_events[i], bs), "join");
     }
     for (std::size_t i = 1; i < branches; ++i) cuda_check(cudaStreamWaitEvent(st, e->branch_events[i], 0), "join wait");
@@ -650,7 +658,7 @@ void enqueue_update(faco_engine* e, cudaStream_t st, const std::uint32_t* list, 
     }
     cuda_check(faco::launch_colony_update(e->d_instances.get(), e->colonies.get(), e->states.get(), v.P,
                                           v.trace_cap ? e->trace.get() : nullptr, list, colonies, v.count,
-                                          v.trace_cap, st),
+                                          v.trace_cap, st, v.overlap),
                "colony update");
     if (v.P.trail_blocks > 1)
         faco::colony_trails_kernel<<<dim3(v.P.trail_blocks, colonies), 256, 0, st>>>(
@@ -671,7 +679,7 @@ void enqueue_chain_iteration(faco_engine* e, std::size_t g, cudaStream_t st) {
     auto& v = e->eval;
     const auto& ch = v.chains[g];
     const auto& c = v.classes[ch.cls];
-    cuda_check(faco::launch_ant_kernel(c.mode, ch.L, ch.blocks, c.warps, c.smem, st), "ant launch");
+    cuda_check(faco::launch_ant_kernel(c.mode, ch.L, ch.blocks, c.warps, c.smem, st, v.overlap), "ant launch");
     enqueue_update(e, st, e->chain_colonies.get() + ch.first, ch.count);
 }
 
@@ -780,6 +788,9 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
     // one wave of the GPU run the build that favours throughput over one
     // ant's latency
     v.full = static_cast<std::uint64_t>(v.count) * A > 32ull * static_cast<std::uint64_t>(e->sm_count);
+    // small panels (at most kOverlapWarps ant warps per SM): blocks that wait
+    // for the kernel before theirs have room beside it
+    v.overlap = static_cast<std::uint64_t>(v.count) * A <= kOverlapWarps * static_cast<std::uint64_t>(e->sm_count);
     v.follow = c.follow != FACO_FOLLOW_OFF;
     v.batch_from = c.follow == FACO_FOLLOW_ON ? 0u : v.full ? kBatchFromFull : kBatchFromOneWave;
     bool need_workspace = false;

@@ -81,6 +81,8 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
         __syncthreads();
         xy = staged;
     }
+    // the previous iteration's update: its parent, trails and state from here on
+    wait_previous_kernel();
     if (!active) return;
 
     node_t* ring = kEngine ? L.colonies[colony].ant_tours + (size_t)ant * L.colonies[colony].n_pad
@@ -403,6 +405,7 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
             for (std::uint32_t i = lane; i < n; i += 32) L.out_construction[(size_t)task * n + i] = s.tour[i];
         __syncwarp();
     }
+    start_next_kernel();   // the update may launch; it waits for the last ant
     // ---------------- local search ----------------
     // (the instance's and the colony's fields are read again where a phase
     // uses them: kept from the start they would hold 20 registers)
@@ -495,11 +498,29 @@ cudaError_t prepare_ant_kernel(int mode, std::uint32_t ls_mode, std::uint32_t sm
     return for_variant(mode, ls_mode, [&](auto m) { return prepare_mode<decltype(m)::value>(smem); });
 }
 
+// Launches `kernel`, with `overlapped` as a programmatic dependent of the
+// kernel before it on the stream: its prologue, up to wait_previous_kernel(),
+// overlaps that kernel.
+template <class... Params, class... Args>
+static cudaError_t launch_overlapped(bool overlapped, void (*kernel)(Params...), std::uint32_t blocks,
+                                     std::uint32_t threads, std::uint32_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(blocks);
+    config.blockDim = dim3(threads);
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &attribute;
+    config.numAttrs = overlapped ? 1 : 0;
+    return cudaLaunchKernelEx(&config, kernel, static_cast<Params>(args)...);
+}
+
 cudaError_t launch_ant_kernel(int mode, const AntLaunch& L, std::uint32_t blocks, std::uint32_t warps,
-                              std::uint32_t smem, cudaStream_t stream) {
+                              std::uint32_t smem, cudaStream_t stream, bool overlapped) {
     return for_variant(mode, L.ls_mode, [&](auto m) {
-        ant_kernel<decltype(m)::value><<<dim3(blocks), dim3(warps * 32), smem, stream>>>(L);
-        return cudaGetLastError();
+        return launch_overlapped(overlapped, ant_kernel<decltype(m)::value>, blocks, warps * 32, smem, stream, L);
     });
 }
 
@@ -1541,6 +1562,8 @@ colony_update_kernel(const InstanceView* instances, const ColonyView* colonies, 
     __shared__ unsigned long long s_steps, s_evals;
     __shared__ std::uint32_t s_used_mne, s_parent_p0;
 
+    start_next_kernel();
+    wait_previous_kernel();
     for (std::uint32_t w = threadIdx.x; w < sizeof(ColonyState) / 4; w += blockDim.x)
         reinterpret_cast<std::uint32_t*>(&s_st)[w] = reinterpret_cast<const std::uint32_t*>(states + c)[w];
     // iteration best: first strict minimum over ants (costs are >= 0); work counters
@@ -1759,12 +1782,11 @@ colony_update_kernel(const InstanceView* instances, const ColonyView* colonies, 
 cudaError_t launch_colony_update(const InstanceView* instances, const ColonyView* colonies, ColonyState* states,
                                  const ColonyParams& P, TraceRow* trace, const std::uint32_t* list,
                                  std::uint32_t blocks, std::uint32_t colony_count, std::uint32_t trace_cap,
-                                 cudaStream_t stream) {
+                                 cudaStream_t stream, bool overlapped) {
     const auto launch = [&](auto control) {
         constexpr int kControl = decltype(control)::value;
-        colony_update_kernel<kControl><<<blocks, update_threads(kControl), 0, stream>>>(
-            instances, colonies, states, P, trace, list, colony_count, trace_cap);
-        return cudaGetLastError();
+        return launch_overlapped(overlapped, colony_update_kernel<kControl>, blocks, update_threads(kControl), 0, stream,
+                                 instances, colonies, states, P, trace, list, colony_count, trace_cap);
     };
     if (P.ref_control) return launch(std::integral_constant<int, 2>{});
     return P.controlled ? launch(std::integral_constant<int, 1>{}) : launch(std::integral_constant<int, 0>{});

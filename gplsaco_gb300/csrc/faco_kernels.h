@@ -56,8 +56,10 @@ cudaError_t launch_knn(const int2* xy, std::uint32_t n, std::uint32_t needed, no
 
 // Host-side launchers (the kernels are defined in faco_kernels.cu).
 cudaError_t prepare_ant_kernel(int mode, std::uint32_t ls_mode, std::uint32_t smem_bytes);
+// (`overlapped`: the kernel's prologue may start while the kernel before it on
+// the stream still runs)
 cudaError_t launch_ant_kernel(int mode, const AntLaunch& L, std::uint32_t blocks, std::uint32_t warps,
-                              std::uint32_t smem_bytes, cudaStream_t stream);
+                              std::uint32_t smem_bytes, cudaStream_t stream, bool overlapped = false);
 
 __global__ void colony_init_kernel(const InstanceView* instances, const ColonyView* colonies, ColonyState* states,
                                    ColonyParams P, std::uint32_t colony_count);
@@ -69,7 +71,7 @@ __global__ void fingerprint_kernel(const ColonyView* colonies, const std::uint32
 cudaError_t launch_colony_update(const InstanceView* instances, const ColonyView* colonies, ColonyState* states,
                                  const ColonyParams& P, TraceRow* trace, const std::uint32_t* list,
                                  std::uint32_t blocks, std::uint32_t colony_count, std::uint32_t trace_cap,
-                                 cudaStream_t stream);
+                                 cudaStream_t stream, bool overlapped = false);
 __global__ void colony_trails_kernel(const InstanceView* instances, const ColonyView* colonies,
                                      const ColonyState* states, ColonyParams P, const std::uint32_t* list);
 __global__ void pheromone_step_kernel(std::uint32_t n, std::uint32_t k, const node_t* primary,

@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(128) mlp_grad_kernel(const MlpParams* P, const
                                                        float inv_count, MlpParams* partials, float* loss_partials,
                                                        unsigned* error) {
     extern __shared__ __align__(16) unsigned char smem[];
-    tc::start_next_kernel();
+    start_next_kernel();
     tc::gradient_rows(
         P, O, E, inv_count, smem, error,
         [&](std::uint32_t row) { return *reinterpret_cast<const uint4*>(x + (size_t)row * kMlpIn); },
@@ -90,8 +90,8 @@ __global__ void __launch_bounds__(128) mlp_step_kernel(const MlpParams* partials
                                                        std::uint32_t blocks, MlpParams* P, MlpOperands* O,
                                                        MlpParams* m, MlpParams* v, float lr, float beta1, float beta2,
                                                        float eps, float bias1, float bias2, float* loss) {
-    tc::start_next_kernel();
-    tc::wait_previous_kernel();
+    start_next_kernel();
+    wait_previous_kernel();
     const float* src = reinterpret_cast<const float*>(partials);
     float* p = reinterpret_cast<float*>(P);
     float* mm = reinterpret_cast<float*>(m);

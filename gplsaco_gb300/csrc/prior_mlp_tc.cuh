@@ -330,12 +330,6 @@ __device__ __forceinline__ uint4 pack8(const float* a) {
     return make_uint4(pack_bf16(a[0], a[1]), pack_bf16(a[2], a[3]), pack_bf16(a[4], a[5]), pack_bf16(a[6], a[7]));
 }
 
-// Programmatic dependent launch: lets the next kernel of the stream start its
-// prologue now; waits until the previous one is complete and its writes are
-// visible (both without effect in an ordinary launch).
-__device__ __forceinline__ void start_next_kernel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void wait_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // Partial gradient and loss sum of this CTA's rows (128-row tiles strided
 // over the grid) into *grad and *loss_sum.  128 threads, `smem` holds
 // kGradSmemBytes (16-byte aligned).  Returns false (and sets
