@@ -210,6 +210,7 @@ struct ColonyView {
     unsigned long long* ant_ids;   // [ants][2] fingerprints of the batch's tours
     std::uint32_t* ant_p0;         // [ants] position of node 0 in each tour
     std::uint32_t* walk;           // construction steps per ant of the last iteration (null: not kept)
+    node_t* parent_pos;            // [n_pad] inverse of `parent` (null: not kept, the ants build their own)
 };
 
 struct TraceRow {

@@ -294,7 +294,7 @@ struct faco_engine {
     DeviceBuffer<faco::InstanceView> d_instances;
     // evaluation buffers (grow-only)
     DeviceBuffer<float> trails, products, colony_eta;
-    DeviceBuffer<faco::node_t> parent, epoch, global, ant_tours;
+    DeviceBuffer<faco::node_t> parent, parent_pos, epoch, global, ant_tours;
     DeviceBuffer<std::uint32_t> parent_nbr;
     DeviceBuffer<long long> ant_costs, ant_ccosts;
     DeviceBuffer<faco::Program> programs;
@@ -1020,6 +1020,7 @@ void begin_evaluation(faco_engine* e, const uint64_t* keys, const uint64_t* seed
     e->products.resize(tau_total);
     e->colony_eta.resize(tau_total);
     e->parent.resize(node_total);
+    e->parent_pos.resize(node_total);
     e->parent_nbr.resize(node_total);
     e->epoch.resize(node_total);
     e->global.resize(node_total);
@@ -1079,6 +1080,8 @@ void begin_evaluation(faco_engine* e, const uint64_t* keys, const uint64_t* seed
         cv.products = e->products.get() + tau_off;
         cv.eta = e->colony_eta.get() + tau_off;
         cv.parent = e->parent.get() + node_off;
+        // (read by the ants of the global-memory workspace)
+        cv.parent_pos = may_use_global(e->settings, in.n) ? e->parent_pos.get() + node_off : nullptr;
         cv.parent_nbr = e->parent_nbr.get() + node_off;
         cv.epoch = e->epoch.get() + node_off;
         cv.global = e->global.get() + node_off;
@@ -1558,6 +1561,17 @@ int faco_restore(faco_engine* e, const void* buffer, uint64_t bytes, uint32_t tr
             put(e->colony_eta.get(), eta, h.tau_total * sizeof(float));
             put(e->parent.get(), parent, h.node_total * sizeof(faco::node_t));
             put(e->parent_nbr.get(), nbr, h.node_total * sizeof(std::uint32_t));
+            // (the parents' inverse is not part of a snapshot)
+            std::vector<faco::node_t> parents(h.node_total), inverse(h.node_total, 0);
+            std::memcpy(parents.data(), parent, h.node_total * sizeof(faco::node_t));
+            for (std::size_t c = 0, off = 0; c < v.sizes.size(); off += faco::pad8(v.sizes[c]), ++c)
+                for (std::uint32_t i = 0; i < v.sizes[c]; ++i) {
+                    const std::uint32_t node = parents[off + i];
+                    require(node < v.sizes[c], "snapshot parent node out of range");
+                    inverse[off + node] = static_cast<faco::node_t>(i);
+                }
+            put(e->parent_pos.get(), reinterpret_cast<const unsigned char*>(inverse.data()),
+                h.node_total * sizeof(faco::node_t));
             put(e->epoch.get(), epoch, h.node_total * sizeof(faco::node_t));
             put(e->global.get(), global, h.node_total * sizeof(faco::node_t));
             require(v.feature_spec == h.feature_spec, "snapshot controller spec differs");

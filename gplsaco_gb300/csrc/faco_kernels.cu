@@ -23,11 +23,22 @@ namespace faco {
 // ---------------------------------------------------------------------------
 // Ant kernel
 // ---------------------------------------------------------------------------
-// Copies a parent tour into the warp's shared tour/inverse.  Engine parents
-// are 16-byte aligned with padded rows, so lanes move 8 nodes per load.
-__device__ __forceinline__ void load_parent(const AntSmem& s, const node_t* parent, std::uint32_t n,
-                                            std::uint32_t lane, bool aligned) {
-    if (aligned) {
+// Copies a parent tour into the warp's tour/inverse.  Engine parents are
+// 16-byte aligned with padded rows, so lanes move 8 nodes per load.  In the
+// global-memory workspace the inverse, which the colony's update writes once,
+// is copied the same way: scattered to global memory by every ant it was an
+// eighth of an ant's time (the large panel 107 -> 90 ms).  In shared memory the
+// scatter is the cheaper one (the uneven batch 82 ms, copied 85).
+__device__ __forceinline__ void load_parent(const AntSmem& s, const node_t* parent, const node_t* inverse,
+                                            std::uint32_t n, std::uint32_t lane, bool aligned) {
+    if (aligned && inverse) {
+        const uint4 *tour = reinterpret_cast<const uint4*>(parent), *pos = reinterpret_cast<const uint4*>(inverse);
+        for (std::uint32_t c = lane; c * 8 < n; c += 32) {
+            const uint4 a = __ldg(tour + c), b = __ldg(pos + c);
+            reinterpret_cast<uint4*>(s.tour)[c] = a;
+            reinterpret_cast<uint4*>(s.pos)[c] = b;
+        }
+    } else if (aligned) {
         const uint4* src = reinterpret_cast<const uint4*>(parent);
         uint4* dst = reinterpret_cast<uint4*>(s.tour);
         for (std::uint32_t c = lane; c * 8 < n; c += 32) {
@@ -118,7 +129,7 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
         cost = L.task_costs[task];
         target = MODE == kModePrepare ? 0 : L.task_targets[task];
     }
-    load_parent(s, parent, n, lane, kEngine);
+    load_parent(s, parent, kGlobalWs ? cv.parent_pos : nullptr, n, lane, kEngine);
     const std::uint32_t words = (n + 31) / 32;
     for (std::uint32_t i = lane; i < words; i += 32) {
         s.visited[i] = 0;
@@ -1397,9 +1408,11 @@ __device__ void ref_decide(const ColonyView& cv, const InstanceView& in, ColonyS
         const node_t* tour = archive_tour(cv, side, alt);
         for (std::uint32_t i = threadIdx.x; i < n; i += blockDim.x) cv.parent[i] = cv.epoch[i] = tour[i];
         __syncthreads();
-        for (std::uint32_t i = threadIdx.x; i < n; i += blockDim.x)
+        for (std::uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
             cv.parent_nbr[cv.parent[i]] = (std::uint32_t)cv.parent[i + 1 == n ? 0 : i + 1] |
                                           ((std::uint32_t)cv.parent[i == 0 ? n - 1 : i - 1] << 16);
+            if (cv.parent_pos) cv.parent_pos[cv.parent[i]] = (node_t)i;
+        }
         const float tmax = st.tau_max;
         for (std::uint32_t i = threadIdx.x; i < n * k; i += blockDim.x) {
             cv.trails[i] = tmax;
@@ -1465,6 +1478,7 @@ __global__ void colony_init_kernel(const InstanceView* instances, const ColonyVi
     for (std::uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
         const node_t v = in.initial[i];
         cv.parent[i] = cv.epoch[i] = cv.global[i] = v;
+        if (cv.parent_pos) cv.parent_pos[v] = (node_t)i;
         cv.parent_nbr[v] = (std::uint32_t)in.initial[i + 1 == n ? 0 : i + 1] |
                            ((std::uint32_t)in.initial[i == 0 ? n - 1 : i - 1] << 16);
     }
@@ -1634,6 +1648,7 @@ colony_update_kernel(const InstanceView* instances, const ColonyView* colonies, 
             if (i >= n) continue;
             const std::uint32_t next = i + 1 == n || u == 7 ? after : (words[(u + 1) >> 1 & 3] >> (16 * ((u + 1) & 1))) & 0xffffu;
             cv.parent_nbr[node] = next | before << 16;
+            if (cv.parent_pos) cv.parent_pos[node] = (node_t)i;
             before = node;
             if (CONTROL == 2 && node == 0) s_parent_p0 = i;
         }
@@ -1759,9 +1774,11 @@ colony_update_kernel(const InstanceView* instances, const ColonyView* colonies, 
             // restart: parent and epoch <- global best, trails <- tau_max
             for (std::uint32_t i = threadIdx.x; i < n; i += blockDim.x) cv.parent[i] = cv.epoch[i] = cv.global[i];
             __syncthreads();
-            for (std::uint32_t i = threadIdx.x; i < n; i += blockDim.x)
+            for (std::uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
                 cv.parent_nbr[cv.parent[i]] = (std::uint32_t)cv.parent[i + 1 == n ? 0 : i + 1] |
                                               ((std::uint32_t)cv.parent[i == 0 ? n - 1 : i - 1] << 16);
+                if (cv.parent_pos) cv.parent_pos[cv.parent[i]] = (node_t)i;
+            }
             const float tmax = s_st.tau_max;
             for (std::uint32_t i = threadIdx.x; i < n * k; i += blockDim.x) {
                 cv.trails[i] = tmax;
