@@ -195,53 +195,90 @@ struct AntResult {
     std::uint32_t limit_reached, checklist;
 };
 
+// Rounds of a shift, reversal or copy taken as one, all loads before the first
+// store.  In the global-memory workspace a round waits for L2: three in one cut
+// the large panel (80 colonies x 64 ants, N 5000-10000) from 90 to 73 ms (two
+// 78; four 78, with spills).  In shared memory the longer code and its
+// registers cost more than the shorter wait (two in one: 256 x 32 ants at
+// N=1000 158 instead of 109 ms).
+template <bool kGlobal>
+constexpr std::uint32_t kRound = kGlobal ? 3u : 1u;
+
 // Moves `node` right after `target` (CpuTour::relocate): shifts the closed
-// interval between their positions by one, register-staged per 64-element
-// chunk (two elements per lane) so that every read of a chunk precedes its
+// interval between their positions by one, register-staged per chunk (two
+// elements per lane and round) so that every read of a chunk precedes its
 // writes; chunks run away from the vacated end.
+template <bool kGlobal>
 __device__ __forceinline__ void relocate_shift(const AntSmem& s, std::uint32_t lane, std::uint32_t tpos,
                                                std::uint32_t npos, std::uint32_t node) {
+    constexpr std::uint32_t kEach = 2 * kRound<kGlobal>;
+    std::uint32_t v[kEach];
     if (tpos < npos) {
         // new[tpos+1] = node, new[i] = old[i-1] for i in (tpos+1, npos]
         const int lo = (int)tpos + 1;
-        for (int base = (int)npos; base >= lo; base -= 64) {
-            const int i0 = base - (int)lane, i1 = i0 - 32;
-            std::uint32_t v0 = 0, v1 = 0;
-            const bool a0 = i0 >= lo, a1 = i1 >= lo;
-            if (a0) v0 = i0 == lo ? node : s.tour[i0 - 1];
-            if (a1) v1 = i1 == lo ? node : s.tour[i1 - 1];
+        for (int base = (int)npos; base >= lo; base -= 32 * (int)kEach) {
+#pragma unroll
+            for (std::uint32_t u = 0; u < kEach; ++u) {
+                const int i = base - (int)lane - 32 * (int)u;
+                if (i >= lo) v[u] = i == lo ? node : s.tour[i - 1];
+            }
             __syncwarp();
-            if (a0) { s.tour[i0] = (node_t)v0; s.pos[v0] = (node_t)i0; }
-            if (a1) { s.tour[i1] = (node_t)v1; s.pos[v1] = (node_t)i1; }
+#pragma unroll
+            for (std::uint32_t u = 0; u < kEach; ++u) {
+                const int i = base - (int)lane - 32 * (int)u;
+                if (i >= lo) { s.tour[i] = (node_t)v[u]; s.pos[v[u]] = (node_t)i; }
+            }
             __syncwarp();
         }
     } else {
         // new[i] = old[i+1] for i in [npos, tpos), new[tpos] = node
-        for (std::uint32_t base = npos; base <= tpos; base += 64) {
-            const std::uint32_t i0 = base + lane, i1 = i0 + 32;
-            std::uint32_t v0 = 0, v1 = 0;
-            const bool a0 = i0 <= tpos, a1 = i1 <= tpos;
-            if (a0) v0 = i0 == tpos ? node : s.tour[i0 + 1];
-            if (a1) v1 = i1 == tpos ? node : s.tour[i1 + 1];
+        for (std::uint32_t base = npos; base <= tpos; base += 32 * kEach) {
+#pragma unroll
+            for (std::uint32_t u = 0; u < kEach; ++u) {
+                const std::uint32_t i = base + lane + 32 * u;
+                if (i <= tpos) v[u] = i == tpos ? node : s.tour[i + 1];
+            }
             __syncwarp();
-            if (a0) { s.tour[i0] = (node_t)v0; s.pos[v0] = (node_t)i0; }
-            if (a1) { s.tour[i1] = (node_t)v1; s.pos[v1] = (node_t)i1; }
+#pragma unroll
+            for (std::uint32_t u = 0; u < kEach; ++u) {
+                const std::uint32_t i = base + lane + 32 * u;
+                if (i <= tpos) { s.tour[i] = (node_t)v[u]; s.pos[v[u]] = (node_t)i; }
+            }
             __syncwarp();
         }
     }
 }
 
-// Reverses tour[lo..hi] (inclusive, lo <= hi, no wrap) with the inverse.
-__device__ __forceinline__ void reverse_range(const AntSmem& s, std::uint32_t lane, std::uint32_t lo,
-                                              std::uint32_t hi) {
-    const std::uint32_t count = hi - lo + 1;
-    for (std::uint32_t o = lane; o < count / 2; o += 32) {
-        const std::uint32_t l = lo + o, r = hi - o;
-        const node_t a = s.tour[l], b = s.tour[r];
-        s.tour[l] = b; s.tour[r] = a;
-        s.pos[b] = (node_t)l; s.pos[a] = (node_t)r;
+// Swaps the pairs (l, r) = ends(o), o in [0, pairs), of disjoint tour
+// positions, with the inverse.
+template <bool kGlobal, class Ends>
+__device__ __forceinline__ void swap_pairs(const AntSmem& s, std::uint32_t lane, std::uint32_t pairs, Ends ends) {
+    constexpr std::uint32_t kEach = kRound<kGlobal>;
+    for (std::uint32_t first = lane; first < pairs; first += 32 * kEach) {
+        node_t a[kEach], b[kEach];
+#pragma unroll
+        for (std::uint32_t u = 0; u < kEach; ++u) {
+            if (first + 32 * u >= pairs) continue;
+            const uint2 at = ends(first + 32 * u);
+            a[u] = s.tour[at.x];
+            b[u] = s.tour[at.y];
+        }
+#pragma unroll
+        for (std::uint32_t u = 0; u < kEach; ++u) {
+            if (first + 32 * u >= pairs) continue;
+            const uint2 at = ends(first + 32 * u);
+            s.tour[at.x] = b[u]; s.tour[at.y] = a[u];
+            s.pos[b[u]] = (node_t)at.x; s.pos[a[u]] = (node_t)at.y;
+        }
     }
     __syncwarp();
+}
+
+// Reverses tour[lo..hi] (inclusive, lo <= hi, no wrap) with the inverse.
+template <bool kGlobal>
+__device__ __forceinline__ void reverse_range(const AntSmem& s, std::uint32_t lane, std::uint32_t lo,
+                                              std::uint32_t hi) {
+    swap_pairs<kGlobal>(s, lane, (hi - lo + 1) / 2, [&](std::uint32_t o) { return uint2{lo + o, hi - o}; });
 }
 
 // A run of relocations deferred during construction.  Once trails converge
@@ -303,9 +340,10 @@ struct RelocationRun {
     }
     // Rewrites the span so that the tour holds the relocated order; the run
     // ends.  `last` is the node taken last (the ant's current node).
+    template <bool kGlobal>
     __device__ void apply(const AntSmem& s, std::uint32_t lane, std::uint32_t last) {
         if (m == 1) {
-            relocate_shift(s, lane, t, p, last);   // reads before its first write, after a warp barrier
+            relocate_shift<kGlobal>(s, lane, t, p, last);   // reads before its first write, after a warp barrier
             m = 0;
             return;
         }
@@ -313,15 +351,15 @@ struct RelocationRun {
         if (p < t) {
             // [sources | span] -> [span | taken in order]
             const std::uint32_t lo = dir > 0 ? p : p - m + 1, span = t - lo + 1 - m;
-            reverse_range(s, lane, lo, t);
-            if (span > 1) reverse_range(s, lane, lo, lo + span - 1);
-            if (dir > 0) reverse_range(s, lane, t - m + 1, t);
+            reverse_range<kGlobal>(s, lane, lo, t);
+            if (span > 1) reverse_range<kGlobal>(s, lane, lo, lo + span - 1);
+            if (dir > 0) reverse_range<kGlobal>(s, lane, t - m + 1, t);
         } else {
             // [span | sources] -> [taken in order | span]
             const std::uint32_t hi = dir > 0 ? p + m - 1 : p, span = hi - t - m;
-            reverse_range(s, lane, t + 1, hi);
-            if (dir > 0) reverse_range(s, lane, t + 1, t + m);
-            if (span > 1) reverse_range(s, lane, t + m + 1, hi);
+            reverse_range<kGlobal>(s, lane, t + 1, hi);
+            if (dir > 0) reverse_range<kGlobal>(s, lane, t + 1, t + m);
+            if (span > 1) reverse_range<kGlobal>(s, lane, t + m + 1, hi);
         }
         m = 0;
     }
@@ -565,6 +603,7 @@ __device__ inline std::uint32_t follow_batch(const AntSmem& s, const int2* xy, c
 // of its two end nodes, as disjoint swap pairs.  Returns the number of
 // elements in the reversed segment.  Every lane has read what it needs of the
 // tour before the call's barrier.
+template <bool kGlobal>
 __device__ __forceinline__ std::uint32_t flip(const AntSmem& s, std::uint32_t n, std::uint32_t lane,
                                               std::uint32_t first, std::uint32_t last) {
     if (first > last) { const std::uint32_t t = first; first = last; last = t; }
@@ -572,15 +611,12 @@ __device__ __forceinline__ std::uint32_t flip(const AntSmem& s, std::uint32_t n,
     const bool straight = length <= n - length || first == 0;
     const std::uint32_t count = straight ? length : n - length, begin = straight ? first : last;
     __syncwarp();
-    for (std::uint32_t o = lane; o < count / 2; o += 32) {
-        std::uint32_t l = begin + o, r = begin + count - 1 - o;
-        if (l >= n) l -= n;
-        if (r >= n) r -= n;
-        const node_t a = s.tour[l], b = s.tour[r];
-        s.tour[l] = b; s.tour[r] = a;
-        s.pos[b] = (node_t)l; s.pos[a] = (node_t)r;
-    }
-    __syncwarp();
+    swap_pairs<kGlobal>(s, lane, count / 2, [&](std::uint32_t o) {
+        uint2 at{begin + o, begin + count - 1 - o};
+        if (at.x >= n) at.x -= n;
+        if (at.y >= n) at.y -= n;
+        return at;
+    });
     return count;
 }
 
@@ -612,6 +648,7 @@ __device__ __forceinline__ std::uint32_t flip(const AntSmem& s, std::uint32_t n,
 // words and the reversal's ends by position: a further 3-6 %.
 constexpr std::uint32_t kPopNodes = 4;
 
+template <bool kGlobal>
 __device__ __forceinline__ void checklist_two_opt(const AntSmem& s, const int2* xy, const InstanceView& in,
                                                   std::uint32_t n, std::uint32_t lane, Checklist& q,
                                                   unsigned long long cap, AntResult& r, long long& gain_sum,
@@ -753,7 +790,7 @@ __device__ __forceinline__ void checklist_two_opt(const AntSmem& s, const int2* 
             // all four ends become pending, in this order; reversed between the first two
             const std::uint32_t m0 = back ? node : close, m1 = back ? bj : nbj;
             const std::uint32_t m2 = back ? close : node, m3 = back ? nbj : bj;
-            r.moved += flip(s, n, lane, p0, p1);
+            r.moved += flip<kGlobal>(s, n, lane, p0, p1);
             r.reactivations += push_lanes(s, q, n, lane == 0 ? m0 : lane == 1 ? m1 : lane == 2 ? m2 : m3, lane < 4,
                                           lane, log, log_cap);
             ++r.accepted;
@@ -783,6 +820,7 @@ __device__ __forceinline__ void checklist_two_opt(const AntSmem& s, const int2* 
 // in the global-memory workspace a pop is a chain of five L2 reads, which the
 // nodes of a pass share.  One GB300, the large panel (80 colonies x 64 ants,
 // N 5000-10000, 80 iterations): 132 -> 110 ms.
+template <bool kGlobal>
 __device__ __forceinline__ void checklist_ls_first(const AntSmem& s, const int2* xy, const InstanceView& in,
                                                    std::uint32_t n, std::uint32_t lane, Checklist& q,
                                                    unsigned long long cap, AntResult& r, long long& gain_sum,
@@ -1009,7 +1047,7 @@ __device__ __forceinline__ void checklist_ls_first(const AntSmem& s, const int2*
             for (std::uint32_t t = 0; t < or_len; ++t) {
                 const std::uint32_t moved = __shfl_sync(kFull, near, own + 1 + (or_side ? or_len - 1 - t : t));
                 const std::uint32_t tp = s.pos[target], np = s.pos[moved];
-                relocate_shift(s, lane, tp, np, moved);
+                relocate_shift<kGlobal>(s, lane, tp, np, moved);
                 r.moved += tp < np ? np - tp : tp - np + 1;
                 target = moved;
             }
@@ -1028,7 +1066,7 @@ __device__ __forceinline__ void checklist_ls_first(const AntSmem& s, const int2*
             const bool back = move_seg & 1u;
             const std::uint32_t m0 = back ? node : close, m1 = back ? move_c : move_nb;
             const std::uint32_t m2 = back ? close : node, m3 = back ? move_nb : move_c;
-            r.moved += flip(s, n, lane, s.pos[m0], s.pos[m1]);
+            r.moved += flip<kGlobal>(s, n, lane, s.pos[m0], s.pos[m1]);
             r.reactivations += push_lanes(s, q, n, lane == 0 ? m0 : lane == 1 ? m1 : lane == 2 ? m2 : m3, lane < 4,
                                           lane, log, log_cap);
             ++r.accepted;

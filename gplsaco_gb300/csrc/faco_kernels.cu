@@ -33,10 +33,23 @@ __device__ __forceinline__ void load_parent(const AntSmem& s, const node_t* pare
                                             std::uint32_t n, std::uint32_t lane, bool aligned) {
     if (aligned && inverse) {
         const uint4 *tour = reinterpret_cast<const uint4*>(parent), *pos = reinterpret_cast<const uint4*>(inverse);
-        for (std::uint32_t c = lane; c * 8 < n; c += 32) {
-            const uint4 a = __ldg(tour + c), b = __ldg(pos + c);
-            reinterpret_cast<uint4*>(s.tour)[c] = a;
-            reinterpret_cast<uint4*>(s.pos)[c] = b;
+        constexpr std::uint32_t kEach = kRound<true>;
+        for (std::uint32_t first = lane; first * 8 < n; first += 32 * kEach) {
+            uint4 a[kEach], b[kEach];
+#pragma unroll
+            for (std::uint32_t u = 0; u < kEach; ++u) {
+                const std::uint32_t c = first + 32 * u;
+                if (c * 8 >= n) continue;
+                a[u] = __ldg(tour + c);
+                b[u] = __ldg(pos + c);
+            }
+#pragma unroll
+            for (std::uint32_t u = 0; u < kEach; ++u) {
+                const std::uint32_t c = first + 32 * u;
+                if (c * 8 >= n) continue;
+                reinterpret_cast<uint4*>(s.tour)[c] = a[u];
+                reinterpret_cast<uint4*>(s.pos)[c] = b[u];
+            }
         }
     } else if (aligned) {
         const uint4* src = reinterpret_cast<const uint4*>(parent);
@@ -354,7 +367,7 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
                         after = run.read(s, npos + 1 == n ? 0 : npos + 1);
                     }
                 } else {
-                    run.apply(s, lane, current);
+                    run.apply<kGlobalWs>(s, lane, current);
                     npos = s.pos[selected];
                 }
             }
@@ -396,7 +409,7 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
                     run.m = 1;
                     run.dir = 1;
                 } else {
-                    relocate_shift(s, lane, tpos, npos, selected);
+                    relocate_shift<kGlobalWs>(s, lane, tpos, npos, selected);
                 }
                 r.moved += tpos < npos ? npos - tpos : tpos - npos + 1;
             }
@@ -410,7 +423,7 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
             current = selected;
             __syncwarp();
         }
-        if (run.m) run.apply(s, lane, current);
+        if (run.m) run.apply<kGlobalWs>(s, lane, current);
         r.construction_cost = cost;
         if (L.out_construction)
             for (std::uint32_t i = lane; i < n; i += 32) L.out_construction[(size_t)task * n + i] = s.tour[i];
@@ -422,8 +435,8 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
     // uses them: kept from the start they would hold 20 registers)
     long long gain_sum = 0;
     const InstanceView ls_in = *in_ptr;
-    if ((MODE & kOrOptOnly) || (!(MODE & kTwoOptOnly) && L.ls_mode == 1)) checklist_ls_first(s, xy, ls_in, n, lane, q, L.ls_limit, r, gain_sum, log, log_cap);
-    else checklist_two_opt(s, xy, ls_in, n, lane, q, L.ls_limit, r, gain_sum, log, log_cap);
+    if ((MODE & kOrOptOnly) || (!(MODE & kTwoOptOnly) && L.ls_mode == 1)) checklist_ls_first<kGlobalWs>(s, xy, ls_in, n, lane, q, L.ls_limit, r, gain_sum, log, log_cap);
+    else checklist_two_opt<kGlobalWs>(s, xy, ls_in, n, lane, q, L.ls_limit, r, gain_sum, log, log_cap);
     r.final_cost = cost + gain_sum;
     r.checklist = q.pushed;
     if (log && q.pushed > log_cap && lane == 0) atomicOr(L.error, kErrQueueOverflow);
@@ -433,7 +446,16 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
         const ColonyView& to = L.colonies[colony];
         uint4* out = reinterpret_cast<uint4*>(to.ant_tours + (size_t)ant * to.n_pad);
         const uint4* src = reinterpret_cast<const uint4*>(s.tour);
-        for (std::uint32_t c = lane; c * 8 < n; c += 32) out[c] = src[c];
+        constexpr std::uint32_t kEach = kRound<kGlobalWs>;
+        for (std::uint32_t first = lane; first * 8 < n; first += 32 * kEach) {
+            uint4 v[kEach];
+#pragma unroll
+            for (std::uint32_t u = 0; u < kEach; ++u)
+                if ((first + 32 * u) * 8 < n) v[u] = src[first + 32 * u];
+#pragma unroll
+            for (std::uint32_t u = 0; u < kEach; ++u)
+                if ((first + 32 * u) * 8 < n) out[first + 32 * u] = v[u];
+        }
         if (lane == 0) {
             to.ant_costs[ant] = r.final_cost;
             to.ant_ccosts[ant] = r.construction_cost;

@@ -18,8 +18,9 @@ namespace faco {
 // iterations, 7 / 8 blocks: 115.4 / 122.3 ms.  4 / 5 / 6 / 7 / 8 blocks, an
 // earlier build of the same steps: the uneven batch (4,096 ant warps) 69.9 /
 // 68.9 / 72.5 / 78.5 / 79.8 ms; 32 x 128 ants at N=537 27.1 / 27.7 / 29.3 /
-// 30.1 / 29.9 ms; one N=100 colony 4.80 / 4.79 / 5.01 / 5.20 / 5.25 ms; the
-// large panel (global-memory workspace, 2-opt) 497 / 504 / 529 / 542 / 542 ms.
+// 30.1 / 29.9 ms; one N=100 colony 4.80 / 4.79 / 5.01 / 5.20 / 5.25 ms.  The
+// large panel (global-memory workspace, 80 x 64 ants, N 5000-10000), 2 / 3 / 4 /
+// 5 / 6 / 7 blocks: 85 / 74 / 73 / 83 / 89 / 92 ms.
 // With Or-opt (more registers) full panels too run 5: 256 x 32 ants at N=1000,
 // 160 iterations, 5 / 6 / 7 blocks: 71.0 / 73.3 / 74.9 ms.
 constexpr std::uint32_t kMaxWarpsPerBlock = 4;
