@@ -22,9 +22,8 @@
 //     prefix sums, so the choice is always the FP64 one (GB300 runs FP64 at
 //     a small fraction of its FP32 rate);
 //   - relocation shifts run as register-staged warp chunks, reversals as
-//     disjoint swap pairs, the best move by __reduce_max/min_sync, and the
-//     LS rows of the next pending node are fetched while the current one is
-//     evaluated.
+//     disjoint swap pairs, the best move by __reduce_max_sync, and the local
+//     search packs the candidates of several pending nodes into one warp pass.
 #pragma once
 
 #include <climits>

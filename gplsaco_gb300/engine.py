@@ -46,7 +46,7 @@ class FixedFacoSettings:
     force_fingerprint_collisions: int = 0   # diagnostic: all 12-feature-controller fingerprints 0
     chains: int = 0         # independent colony chains per graph (0 auto); results do not depend on it
     follow: int = 0         # 0 auto, 1 off, 2 on: parent-following construction steps in batches
-                            # (auto: when every ant warp fits in one wave); results do not depend on it
+                            # (auto: colonies whose ants walked far); results do not depend on it
 
     def to_c(self) -> _lib.Settings:
         s = _lib.Settings()

@@ -12,9 +12,10 @@ tuner off (so that no tuning launches precede it), restores the snapshot and
 runs L iterations with every kernel launched alone (unchained), printing the
 device milliseconds of the ant kernel and of the colony update.  Under a
 profiler the L ant launches of the second form are the only ant-kernel
-launches of their variant after registration: `ant_kernel<0>` (steps one at
-a time, F=1) or `ant_kernel<7>` (parent-following steps in batches, F=2: the
-batched build for panels beyond one wave, which this panel is).
+launches after registration (`ant_kernel<3>`): `ant_kernel<16>` with F=1
+(steps one at a time) or `ant_kernel<23>` with F=0 (each colony chooses between
+single and batched steps by its last walk; the first iteration after a restore
+knows none and takes single steps) and F=2 (always batches).
 """
 from __future__ import annotations
 
@@ -44,7 +45,7 @@ def main(argv=None) -> None:
     ap.add_argument("--save")
     ap.add_argument("--load")
     ap.add_argument("--iterations", type=int, default=400)
-    ap.add_argument("--follow", type=int, default=1, choices=[1, 2])
+    ap.add_argument("--follow", type=int, default=0, choices=[0, 1, 2])
     ap.add_argument("--launches", type=int, default=1)
     args = ap.parse_args(argv)
     if args.save:
