@@ -432,7 +432,7 @@ __device__ __forceinline__ bool follow_takes(const AntSmem& s, const node_t* row
             const float4 pg = p;
             if (g < k / 4) {
                 x = __ldg(rows + g);
-                p = __ldg(weights + g);
+                p = load_written(weights + g);
             }
             add(xg.x & 0xffffu, pg.x);
             add(xg.x >> 16, pg.y);
@@ -441,7 +441,7 @@ __device__ __forceinline__ bool follow_takes(const AntSmem& s, const node_t* row
         }
     } else {
 #pragma unroll 1
-        for (std::uint32_t j = 0; j < k; ++j) add(__ldg(row + j), __ldg(prow + j));
+        for (std::uint32_t j = 0; j < k; ++j) add(__ldg(row + j), load_written(prow + j));
     }
     if (!(total >= 0x1p-100f)) return false;
     const float threshold = uf * total, delta = total * 0x1p-17f;
@@ -480,7 +480,7 @@ __device__ inline std::uint32_t follow_batch(const AntSmem& s, const int2* xy, c
         t = (int)run.t;
         D = m0 >= 2 ? run.dir : (half ? -1 : 1);
     } else {
-        const std::uint32_t pn = __ldg(parent_nbr + current);
+        const std::uint32_t pn = load_written(parent_nbr + current);
         const std::uint32_t y = half ? pn >> 16 : pn & 0xffffu;
         t0 = s.pos[current];
         const std::uint32_t ty = s.pos[y];
@@ -519,10 +519,10 @@ __device__ inline std::uint32_t follow_batch(const AntSmem& s, const int2* xy, c
     float4 p4 = {0.0f, 0.0f, 0.0f, 0.0f};
     if ((k & 3u) == 0) {
         x = __ldg(reinterpret_cast<const uint2*>(row));
-        p4 = __ldg(reinterpret_cast<const float4*>(prow));
+        p4 = load_written(reinterpret_cast<const float4*>(prow));
     }
     if (ok) {
-        const std::uint32_t pn = __ldg(parent_nbr + cur);
+        const std::uint32_t pn = load_written(parent_nbr + cur);
         ok = (sel == (pn & 0xffffu) || sel == (pn >> 16)) && !test_bit(s.visited, sel);
     }
     // the run as it stands before this lane's step (m = mr): a step onto the

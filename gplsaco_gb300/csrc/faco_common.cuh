@@ -73,6 +73,18 @@ __device__ __forceinline__ void wait_previous_kernel() {
 #endif
 }
 
+// A load of what another kernel of the stream writes while this one may already
+// be resident (a colony's parent, neighbours and products).  Not by __ldg: that
+// is for memory constant over the kernel's life, so it may move above
+// wait_previous_kernel() and need not see the writes.
+template <class T>
+__device__ __forceinline__ T load_written(const T* p) {
+#ifdef __CUDACC__
+    __builtin_assume(__isGlobal(p));   // ld.global, not a generic load
+#endif
+    return *p;
+}
+
 // Philox4x32 with 10 rounds (Salmon, Moraes, Dror, Shaw, SC'11).
 struct uint4v { std::uint32_t x, y, z, w; };
 __device__ __forceinline__ uint4v philox4x32(std::uint32_t c0, std::uint32_t c1, std::uint32_t c2,

@@ -40,8 +40,8 @@ __device__ __forceinline__ void load_parent(const AntSmem& s, const node_t* pare
             for (std::uint32_t u = 0; u < kEach; ++u) {
                 const std::uint32_t c = first + 32 * u;
                 if (c * 8 >= n) continue;
-                a[u] = __ldg(tour + c);
-                b[u] = __ldg(pos + c);
+                a[u] = load_written(tour + c);
+                b[u] = load_written(pos + c);
             }
 #pragma unroll
             for (std::uint32_t u = 0; u < kEach; ++u) {
@@ -55,7 +55,7 @@ __device__ __forceinline__ void load_parent(const AntSmem& s, const node_t* pare
         const uint4* src = reinterpret_cast<const uint4*>(parent);
         uint4* dst = reinterpret_cast<uint4*>(s.tour);
         for (std::uint32_t c = lane; c * 8 < n; c += 32) {
-            const uint4 v = __ldg(src + c);
+            const uint4 v = load_written(src + c);
             dst[c] = v;
             const std::uint32_t words[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -221,21 +221,21 @@ __global__ void __launch_bounds__(kMaxWarpsPerBlock * 32, kAntBlocksPerSM) ant_k
                 cand = next_cand;
                 p = next_p;
             } else {
-                pnbr = __ldg(parent_nbr + current);
+                pnbr = load_written(parent_nbr + current);
                 if (MODE != kModeVisits && lane < k) {
                     cand = __ldg(in.primary + (size_t)current * k + lane);
-                    p = __ldg(products + (size_t)current * k + lane);
+                    p = load_written(products + (size_t)current * k + lane);
                 }
             }
             if (kEngine) {
                 const std::uint32_t ps = pnbr & 0xffffu;
                 next_node = test_bit(s.visited, ps) ? pnbr >> 16 : ps;
-                next_pnbr = __ldg(parent_nbr + next_node);
+                next_pnbr = load_written(parent_nbr + next_node);
                 next_cand = n;
                 next_p = 0.0f;
                 if (lane < k) {
                     next_cand = __ldg(in.primary + (size_t)next_node * k + lane);
-                    next_p = __ldg(products + (size_t)next_node * k + lane);
+                    next_p = load_written(products + (size_t)next_node * k + lane);
                 }
             }
             std::uint32_t selected = n;
