@@ -1567,15 +1567,22 @@ int faco_restore(faco_engine* e, const void* buffer, uint64_t bytes, uint32_t tr
             put(e->colony_eta.get(), eta, h.tau_total * sizeof(float));
             put(e->parent.get(), parent, h.node_total * sizeof(faco::node_t));
             put(e->parent_nbr.get(), nbr, h.node_total * sizeof(std::uint32_t));
-            // (the parents' inverse is not part of a snapshot)
-            std::vector<faco::node_t> parents(h.node_total), inverse(h.node_total, 0);
-            std::memcpy(parents.data(), parent, h.node_total * sizeof(faco::node_t));
-            for (std::size_t c = 0, off = 0; c < v.sizes.size(); off += faco::pad8(v.sizes[c]), ++c)
-                for (std::uint32_t i = 0; i < v.sizes[c]; ++i) {
-                    const std::uint32_t node = parents[off + i];
-                    require(node < v.sizes[c], "snapshot parent node out of range");
-                    inverse[off + node] = static_cast<faco::node_t>(i);
-                }
+            // every tour a permutation, the parent's neighbours its own: the
+            // ants index by them unchecked.  (The parents' inverse is not part
+            // of a snapshot.)
+            std::vector<faco::node_t> tour(h.node_total), inverse(h.node_total, 0);
+            std::vector<std::uint32_t> near(h.node_total);
+            std::memcpy(near.data(), nbr, near.size() * sizeof(std::uint32_t));
+            for (const unsigned char* row : {epoch, global, parent}) {   // the parent last: its inverse stays
+                std::memcpy(tour.data(), row, tour.size() * sizeof(faco::node_t));
+                for (std::size_t c = 0, at = 0; c < v.sizes.size(); at += faco::pad8(v.sizes[c]), ++c)
+                    if (!faco::host_inverse(&tour[at], v.sizes[c], &inverse[at]))
+                        throw Error(FACO_EINVAL, "snapshot tour is not a permutation");
+            }
+            for (std::size_t c = 0, at = 0; c < v.sizes.size(); at += faco::pad8(v.sizes[c]), ++c)
+                for (std::uint32_t i = 0, n = v.sizes[c], before = tour[at + n - 1]; i < n; before = tour[at + i++])
+                    if (near[at + tour[at + i]] != (tour[at + (i + 1 == n ? 0 : i + 1)] | before << 16))
+                        throw Error(FACO_EINVAL, "snapshot parent neighbours differ from the parent tour");
             put(e->parent_pos.get(), reinterpret_cast<const unsigned char*>(inverse.data()),
                 h.node_total * sizeof(faco::node_t));
             put(e->epoch.get(), epoch, h.node_total * sizeof(faco::node_t));

@@ -34,5 +34,8 @@ void host_alpha(const std::vector<std::int32_t>& xy, std::uint32_t n, std::uint3
 void host_distance_order(const std::vector<std::int32_t>& xy, std::uint32_t n, std::uint32_t w,
                          const std::uint32_t* rows, std::vector<std::uint16_t>& ls,
                          std::vector<std::int32_t>& ls_dist);
+// The inverse of a tour (n below 65535): inverse[order[i]] = i.  False where
+// `order` is not a permutation of 0 .. n-1.
+bool host_inverse(const std::uint16_t* order, std::uint32_t n, std::uint16_t* inverse);
 
 }  // namespace faco

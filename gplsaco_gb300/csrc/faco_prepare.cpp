@@ -216,6 +216,16 @@ void host_distance_order(const std::vector<std::int32_t>& xy, std::uint32_t n, s
     }
 }
 
+bool host_inverse(const std::uint16_t* order, std::uint32_t n, std::uint16_t* inverse) {
+    constexpr std::uint16_t kNone = 0xffff;   // no position: n is below it
+    std::fill(inverse, inverse + n, kNone);
+    for (std::uint32_t i = 0; i < n; ++i) {
+        if (order[i] >= n || inverse[order[i]] != kNone) return false;
+        inverse[order[i]] = static_cast<std::uint16_t>(i);
+    }
+    return true;
+}
+
 }  // namespace faco
 
 namespace faco {

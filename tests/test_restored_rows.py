@@ -1,0 +1,92 @@
+"""What a restore takes from a snapshot besides copying it: the inverse of each
+tour, built only for a permutation (on the CPU, from the engine's own host
+source), and the refusal of a snapshot whose tours or parent neighbours could
+not be a colony's, checksum and all else being right."""
+import ctypes as C
+import struct
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+from tests import _cases
+
+CSRC = Path(__file__).resolve().parents[1] / "gplsaco_gb300" / "csrc"
+
+ENTRY = """
+#include "faco_host.h"
+extern "C" int inverse_of(const unsigned short* order, unsigned n, unsigned short* out) {
+    return faco::host_inverse(order, n, out);
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def inverse_of(tmp_path_factory):
+    at = tmp_path_factory.mktemp("inverse")
+    (at / "entry.cpp").write_text(ENTRY)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", f"-I{CSRC}", str(at / "entry.cpp"),
+                    str(CSRC / "faco_prepare.cpp"), "-o", str(at / "inverse.so")], check=True)
+    return C.CDLL(str(at / "inverse.so")).inverse_of
+
+
+@pytest.mark.parametrize("n", [3, 8, 1000, 10000])
+def test_inverse_only_of_a_permutation(inverse_of, n):
+    def call(order):
+        order, out = np.ascontiguousarray(order, np.uint16), np.zeros(n, np.uint16)
+        return inverse_of(order.ctypes.data_as(C.c_void_p), n, out.ctypes.data_as(C.c_void_p)), out
+
+    rng = np.random.default_rng(n)
+    for order in (np.arange(n), np.arange(n)[::-1], rng.permutation(n)):
+        ok, out = call(order)
+        assert ok and np.array_equal(out, np.argsort(order))
+        for at, value in ((0, order[1]), (n - 1, order[0]), (n // 2, n), (1, 0xffff)):
+            broken = order.copy()
+            broken[at] = value   # a node twice, or one beyond the last
+            assert not call(broken)[0]
+
+
+def _fnv1a(data: bytes) -> int:
+    h = 1469598103934665603
+    for byte in data:
+        h = ((h ^ byte) * 1099511628211) & (2**64 - 1)
+    return h
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("workspace", [1, 2])
+def test_broken_rows_are_refused(engine_lib, workspace):
+    import gplsaco_gb300 as g
+    n, colonies = 21, 2
+    keys, seeds = np.array([4, 4], np.uint64), np.array([1, 2], np.uint64)
+    e = g.FacoBatchEngine(n, colonies, g.FixedFacoSettings(ants=9, retention=0.9, workspace=workspace))
+    e.register_problem(4, _cases.uniform_instance(n, seed=3).astype(np.float64))
+    e.begin(keys, seeds, 8)
+    e.step(6)
+    state = e.capture_state().to_bytes()
+    e.step(7)
+    want = e.finish()
+    # the closing rows: parent, neighbours, epoch best, global best, checksum
+    pad = (n + 7) // 8 * 8
+    total = colonies * pad
+    ends = np.cumsum([0, 2 * total, 4 * total, 2 * total, 2 * total])
+    base = len(state) - 8 - int(ends[-1])
+    row = {name: base + int(at) for name, at in zip(("parent", "near", "epoch", "global"), ends)}
+    for name, size in (("parent", 2), ("epoch", 2), ("global", 2), ("near", 4)):
+        for colony in range(colonies):
+            for value in ("other", n):
+                broken = bytearray(state[:-8])
+                at = row[name] + size * (colony * pad + n // 2)
+                other = bytes(broken[at - size:at])
+                broken[at:at + size] = other if value == "other" else struct.pack("<H" if size == 2 else "<I", value)
+                broken += struct.pack("<Q", _fnv1a(broken))
+                with pytest.raises(ValueError, match="snapshot"):
+                    e.restore_state(g.CountedState(bytes(broken)))
+    # and the engine goes on from the sound one
+    e.restore_state(g.CountedState(state))
+    e.step(7)
+    got = e.finish()
+    assert np.array_equal(got["costs"], want["costs"])
+    assert all(np.array_equal(a, b) for a, b in zip(got["tours"], want["tours"]))
+    e.close()
