@@ -1562,6 +1562,13 @@ int faco_restore(faco_engine* e, const void* buffer, uint64_t bytes, uint32_t tr
                 cuda_check(cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, s), "snapshot upload");
             };
             put(e->states.get(), states, h.count * sizeof(faco::ColonyState));
+            std::vector<std::uint32_t> walks(h.count);
+            for (std::uint32_t c = 0; c < h.count; ++c) {
+                faco::ColonyState st;
+                std::memcpy(&st, states + c * sizeof st, sizeof st);
+                walks[c] = faco::host_mean_walk(st.construction_steps, st.iteration, h.ants);
+            }
+            e->walks.upload(walks, s);
             put(e->trails.get(), trails, h.tau_total * sizeof(float));
             put(e->products.get(), products, h.tau_total * sizeof(float));
             put(e->colony_eta.get(), eta, h.tau_total * sizeof(float));

@@ -37,5 +37,9 @@ void host_distance_order(const std::vector<std::int32_t>& xy, std::uint32_t n, s
 // The inverse of a tour (n below 65535): inverse[order[i]] = i.  False where
 // `order` is not a permutation of 0 .. n-1.
 bool host_inverse(const std::uint16_t* order, std::uint32_t n, std::uint16_t* inverse);
+// Construction steps per ant and iteration of a colony's run so far: what a
+// restored colony starts from in place of its last iteration's walk, which a
+// snapshot does not hold.
+std::uint32_t host_mean_walk(std::uint64_t construction_steps, std::uint32_t iterations, std::uint32_t ants);
 
 }  // namespace faco

@@ -226,6 +226,11 @@ bool host_inverse(const std::uint16_t* order, std::uint32_t n, std::uint16_t* in
     return true;
 }
 
+std::uint32_t host_mean_walk(std::uint64_t construction_steps, std::uint32_t iterations, std::uint32_t ants) {
+    const std::uint64_t tours = static_cast<std::uint64_t>(iterations) * ants;
+    return tours ? static_cast<std::uint32_t>(construction_steps / tours) : 0u;
+}
+
 }  // namespace faco
 
 namespace faco {

@@ -14,8 +14,8 @@ device milliseconds of the ant kernel and of the colony update.  Under a
 profiler the L ant launches of the second form are the only ant-kernel
 launches after registration (`ant_kernel<3>`): `ant_kernel<16>` with F=1
 (steps one at a time) or `ant_kernel<23>` with F=0 (each colony chooses between
-single and batched steps by its last walk; the first iteration after a restore
-knows none and takes single steps) and F=2 (always batches).
+single and batched steps by its last walk, after a restore by the mean walk of
+its run so far) and F=2 (always batches).
 """
 from __future__ import annotations
 

@@ -1,7 +1,8 @@
 """What a restore takes from a snapshot besides copying it: the inverse of each
 tour, built only for a permutation (on the CPU, from the engine's own host
-source), and the refusal of a snapshot whose tours or parent neighbours could
-not be a colony's, checksum and all else being right."""
+source), the walk that its colonies start from, and the refusal of a snapshot
+whose tours or parent neighbours could not be a colony's, checksum and all else
+being right."""
 import ctypes as C
 import struct
 import subprocess
@@ -19,23 +20,26 @@ ENTRY = """
 extern "C" int inverse_of(const unsigned short* order, unsigned n, unsigned short* out) {
     return faco::host_inverse(order, n, out);
 }
+extern "C" unsigned mean_walk(unsigned long long steps, unsigned iterations, unsigned ants) {
+    return faco::host_mean_walk(steps, iterations, ants);
+}
 """
 
 
 @pytest.fixture(scope="module")
-def inverse_of(tmp_path_factory):
-    at = tmp_path_factory.mktemp("inverse")
+def host(tmp_path_factory):
+    at = tmp_path_factory.mktemp("host")
     (at / "entry.cpp").write_text(ENTRY)
     subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", f"-I{CSRC}", str(at / "entry.cpp"),
-                    str(CSRC / "faco_prepare.cpp"), "-o", str(at / "inverse.so")], check=True)
-    return C.CDLL(str(at / "inverse.so")).inverse_of
+                    str(CSRC / "faco_prepare.cpp"), "-o", str(at / "host.so")], check=True)
+    return C.CDLL(str(at / "host.so"))
 
 
 @pytest.mark.parametrize("n", [3, 8, 1000, 10000])
-def test_inverse_only_of_a_permutation(inverse_of, n):
+def test_inverse_only_of_a_permutation(host, n):
     def call(order):
         order, out = np.ascontiguousarray(order, np.uint16), np.zeros(n, np.uint16)
-        return inverse_of(order.ctypes.data_as(C.c_void_p), n, out.ctypes.data_as(C.c_void_p)), out
+        return host.inverse_of(order.ctypes.data_as(C.c_void_p), n, out.ctypes.data_as(C.c_void_p)), out
 
     rng = np.random.default_rng(n)
     for order in (np.arange(n), np.arange(n)[::-1], rng.permutation(n)):
@@ -45,6 +49,14 @@ def test_inverse_only_of_a_permutation(inverse_of, n):
             broken = order.copy()
             broken[at] = value   # a node twice, or one beyond the last
             assert not call(broken)[0]
+
+
+@pytest.mark.parametrize("steps,iterations,ants,walk", [(0, 0, 32, 0), (32 * 7, 1, 32, 7), (32 * 400 * 61 + 5, 400, 32, 61),
+                                                        (9999 * 4096 * 2**32 - 1, 2**32 - 1, 4096, 9999)])
+def test_walk_of_a_restored_colony(host, steps, iterations, ants, walk):
+    host.mean_walk.argtypes = [C.c_ulonglong, C.c_uint, C.c_uint]
+    host.mean_walk.restype = C.c_uint
+    assert host.mean_walk(steps, iterations, ants) == walk
 
 
 def _fnv1a(data: bytes) -> int:
