@@ -34,16 +34,6 @@ thread_local std::string g_error;
 
 // Iterations captured per CUDA graph (replayed until the budget is spent).
 constexpr std::uint32_t kGraphIterations = 16;
-// FACO_FOLLOW_AUTO: a colony takes parent-following steps in batches from
-// this many construction steps per ant on, as walked in its last iteration
-// (the ant kernel reads it); below, the batches' setup costs more than the
-// few steps they take at once.  Measured in us per iteration, one at a time /
-// in batches: the uneven batch (4,096 ant warps) 179 / 211 at 23 steps, 224 /
-// 226 at 31, 297 / 251 at 44; 256 x 32 ants at N=1000 340 / 416 at 33 steps,
-// 438 / 448 at 51, 601 / 500 at 80; the large panel in the global-memory
-// workspace (2-opt) 1814 / 1857 at 54, 2195 / 1994 at 80.  Moving a line by a
-// fifth either way changes a run by less than 1 %.
-constexpr std::uint32_t kBatchFromOneWave = 30, kBatchFromFull = 48, kBatchFromGlobal = 60;
 // Up to this many ant warps per SM the iteration's kernels launch as
 // programmatic dependents: one N=100 colony (64 ants) 4.62 -> 4.46 ms, 32 x 32
 // ants with a prior 10.6 -> 9.9 ms.  Beyond, the waiting blocks keep other
@@ -367,7 +357,6 @@ struct faco_engine {
         cudaGraphExec_t exec = nullptr;
         bool full = false;                      // more ant warps than one wave of the GPU
         bool overlap = false;                   // each kernel's prologue overlaps the kernel before it
-        std::uint32_t batch_from = 0;           // AntLaunch::batch_from
     } eval;
     std::vector<cudaStream_t> branch_streams;
     std::vector<cudaEvent_t> branch_events;   // [0] fork, [1 + i] join of branch i
@@ -788,15 +777,14 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
         return jobs;
     };
     // batched parent-following steps (the same results): always on request,
-    // else per colony from its walk length; panels with more ant warps than
-    // one wave of the GPU run the build that favours throughput over one
-    // ant's latency
+    // else per colony from its walk length (host_batch_from); panels with more
+    // ant warps than one wave of the GPU run the build that favours throughput
+    // over one ant's latency
     v.full = static_cast<std::uint64_t>(v.count) * A > 32ull * static_cast<std::uint64_t>(e->sm_count);
     // small panels (at most kOverlapWarps ant warps per SM): blocks that wait
     // for the kernel before theirs have room beside it
     v.overlap = static_cast<std::uint64_t>(v.count) * A <= kOverlapWarps * static_cast<std::uint64_t>(e->sm_count);
     v.follow = c.follow != FACO_FOLLOW_OFF;
-    v.batch_from = c.follow == FACO_FOLLOW_ON ? 0u : v.full ? kBatchFromFull : kBatchFromOneWave;
     bool need_workspace = false;
     for (const auto& cl : v.classes) need_workspace = need_workspace || may_use_global(c, cl.n_max);
     if (need_workspace) e->ant_workspace.resize(2 * e->ant_tours.size());
@@ -810,14 +798,14 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
             cl.warps = std::min<std::uint32_t>(faco::kMaxWarpsPerBlock, std::max(1u, A));
         }
     }
-    auto launch_of = [&](std::uint32_t first_job, std::uint32_t warps, std::uint32_t n_max) {
+    auto launch_of = [&](int mode, std::uint32_t first_job, std::uint32_t warps, std::uint32_t n_max) {
         faco::AntLaunch L = v.L;
         L.work = e->work.get() + first_job;
         L.warps = warps;
         L.n_max = n_max;
         L.workspace = need_workspace ? e->ant_workspace.get() : nullptr;
         L.ant_tours_base = e->ant_tours.get();
-        L.batch_from = v.batch_from;
+        L.batch_from = faco::host_batch_from(c.follow == FACO_FOLLOW_ON, v.full, faco::global_mode(mode));
         return L;
     };
     if (c.autotune) {
@@ -848,7 +836,7 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
                     if (smem > 227u * 1024u) break;
                     const auto jobs = jobs_for(members[i], w);
                     e->work.upload(jobs, s);
-                    const faco::AntLaunch L = launch_of(0, w, cl.n_max);
+                    const faco::AntLaunch L = launch_of(mode, 0, w, cl.n_max);
                     cuda_check(faco::prepare_ant_kernel(timed, c.ls_mode, smem), "attribute");
                     float ms = 0.0f;
                     for (int rep = 0; rep < 3; ++rep) {
@@ -916,20 +904,20 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
         else e->chain_colonies.upload(list, s);
     }
     e->work.upload(all, s);
-    if (v.batch_from)
-        for (const auto& cl : v.classes)
-            if (faco::global_mode(cl.mode)) v.batch_from = kBatchFromGlobal;
     if (v.follow)
         for (auto& cl : v.classes) cl.mode = faco::with_follow(cl.mode, v.full);
     // the dynamic shared-memory limit is a property of each kernel variant,
     // shared by every class that uses it: it must admit the largest one
     std::map<int, std::uint32_t> smem_max;
     for (auto& cl : v.classes) {
-        cl.L = launch_of(cl.first_job, cl.warps, cl.n_max);
+        cl.L = launch_of(cl.mode, cl.first_job, cl.warps, cl.n_max);
         auto& m = smem_max[cl.mode];
         m = std::max(m, cl.smem);
     }
-    for (auto& ch : v.chains) ch.L = launch_of(ch.first_job, v.classes[ch.cls].warps, v.classes[ch.cls].n_max);
+    for (auto& ch : v.chains) {
+        const auto& cl = v.classes[ch.cls];
+        ch.L = launch_of(cl.mode, ch.first_job, cl.warps, cl.n_max);
+    }
     for (const auto& [mode, smem] : smem_max)
         if (smem) cuda_check(faco::prepare_ant_kernel(mode, c.ls_mode, smem), "cudaFuncSetAttribute");
 }
@@ -1674,7 +1662,7 @@ int faco_get_launch_plan(faco_engine* e, faco_launch_plan* plan) {
         plan->chains = chains;
         plan->graph_iterations = kGraphIterations;
         plan->launches_per_iteration = chains ? chains * (1 + per_update) : plan->size_classes + per_update;
-        plan->follow = !v.follow ? 0u : v.full && v.batch_from ? 2u : 1u;
+        plan->follow = !v.follow ? 0u : v.full && e->settings.follow == FACO_FOLLOW_AUTO ? 2u : 1u;
     });
 }
 

@@ -42,4 +42,21 @@ bool host_inverse(const std::uint16_t* order, std::uint32_t n, std::uint16_t* in
 // snapshot does not hold.
 std::uint32_t host_mean_walk(std::uint64_t construction_steps, std::uint32_t iterations, std::uint32_t ants);
 
+// The construction steps per ant from which a colony takes parent-following
+// steps in batches (FACO_FOLLOW_AUTO), as walked in its last iteration (the
+// ant kernel reads it); below, the batches' setup costs more than the few
+// steps they take at once.  A line per launch, by the placement of its own
+// ants: one line for all, the highest, kept the small instances of a mixed
+// panel on single steps (256 x 32 ants of N 500-2500, 200 iterations: 115.4
+// ms, now 113.4).  Measured in us per iteration, one at a time / in
+// batches: the uneven batch (4,096 ant warps) 179 / 211 at 23 steps, 224 /
+// 226 at 31, 297 / 251 at 44; 256 x 32 ants at N=1000 340 / 416 at 33 steps,
+// 438 / 448 at 51, 601 / 500 at 80; the large panel in the global-memory
+// workspace (2-opt) 1814 / 1857 at 54, 2195 / 1994 at 80.
+constexpr std::uint32_t kBatchFromOneWave = 30, kBatchFromFull = 48, kBatchFromGlobal = 60;
+// `always`: FACO_FOLLOW_ON; `full`: more ant warps than one wave of the GPU.
+constexpr std::uint32_t host_batch_from(bool always, bool full, bool global_workspace) {
+    return always ? 0u : global_workspace ? kBatchFromGlobal : full ? kBatchFromFull : kBatchFromOneWave;
+}
+
 }  // namespace faco
