@@ -737,13 +737,6 @@ void capture_graph(faco_engine* e, cudaStream_t st) {
 // run a full block per SM slot instead of one or two shared-memory-bound ants.
 constexpr std::uint32_t kGlobalWorkspaceFrom = 2048;   // auto: n_max above this may use it
 
-// A full panel's shared-memory blocks of that size hold an SM each, which a
-// class timed alone does not show but the other chains do: at N 5000-8166
-// (40 colonies x 64 ants) shared memory timed 0-11 % faster than the global
-// workspace in five panels, and the two panels that took it ran 120 instead of
-// 107 ms; at N 2300-2500 it timed 29 % faster and ran 51 instead of 67 ms.
-constexpr float kSharedHandicap = 1.15f;
-
 bool may_use_global(const faco_settings& c, std::uint32_t n_max) {
     return c.workspace == FACO_WORKSPACE_GLOBAL ||
            (c.workspace == FACO_WORKSPACE_AUTO && n_max > kGlobalWorkspaceFrom);
@@ -849,7 +842,9 @@ void build_work_tables(faco_engine* e, const std::vector<std::vector<std::uint32
                         cuda_check(cudaEventElapsedTime(&one, t0, t1), "elapsed");
                         if (rep > 0) ms += one;   // first launch warms caches
                     }
-                    if (v.full && mode == faco::kModeEngine && may_use_global(c, cl.n_max)) ms *= kSharedHandicap;
+                    if (mode == faco::kModeEngine && may_use_global(c, cl.n_max))
+                        ms *= faco::host_shared_factor(
+                            v.full, faco::block_smem_bytes(cl.n_max, faco::kMaxWarpsPerBlock));
                     if (best_ms == 0.0f || ms < best_ms) {
                         best_ms = ms;
                         cl.warps = w;

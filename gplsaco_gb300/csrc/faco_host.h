@@ -59,4 +59,24 @@ constexpr std::uint32_t host_batch_from(bool always, bool full, bool global_work
     return always ? 0u : global_workspace ? kBatchFromGlobal : full ? kBatchFromFull : kBatchFromOneWave;
 }
 
+// The factor on a class's time with its ants in shared memory, against the
+// global-memory workspace, when the tuner compares the two: it times a class
+// alone, from the initial tours, and a full panel's other chains change which
+// is faster.  By the blocks of four ants that fit on an SM (228 KB, 1 KB of it
+// the driver's per block):
+//   3 and more (N up to about 3,300): nearly as many ants as the workspace's
+//     registers admit, without its L2 reads.  60 iterations of 80 x 64 ants at
+//     N=2200 / 2600 / 3000: 12.3 / 14.8 / 15.7 ms in shared memory, 17.8 / 19.0
+//     / 19.9 in the workspace; the ants above N=2048 of 256 x 32 with N 500-2500
+//     timed the same in both, and the panel ran 81 or 115 ms.
+//   2: alike in a panel of one size (N=3500 / 4000 / 4500: 21.4 / 22.8 / 23.7 ms,
+//     in the workspace 21.2 / 22.3 / 24.0); 120 x 64 ants of N 3773-4485, timed
+//     faster in shared memory, ran 37.3 instead of 32.4 ms.
+//   1 (N from about 4,600 on): a block holds the SM.  At N 5000-8166 (40
+//     colonies x 64 ants) shared memory timed 0-11 % faster than the workspace
+//     in five panels, and the two panels that took it ran 120 instead of 107 ms.
+constexpr float host_shared_factor(bool full, std::uint32_t block_bytes) {
+    return !full ? 1.0f : 3 * (block_bytes + 1024u) <= 228u * 1024u ? 0.8f : 1.15f;
+}
+
 }  // namespace faco

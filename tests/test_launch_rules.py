@@ -16,6 +16,7 @@ ENTRY = """
 extern "C" unsigned batch_from(int always, int full, int global_workspace) {
     return faco::host_batch_from(always, full, global_workspace);
 }
+extern "C" float shared_factor(int full, unsigned block_bytes) { return faco::host_shared_factor(full, block_bytes); }
 """
 
 
@@ -34,6 +35,19 @@ def test_batch_line_is_that_of_the_launch(host):
         for workspace in (0, 1):
             assert host.batch_from(1, full, workspace) == 0
     assert host.batch_from(0, 0, 0) < host.batch_from(0, 1, 0) < host.batch_from(0, 0, 1) == host.batch_from(0, 1, 1)
+
+
+@pytest.mark.parametrize("n,sign", [(2049, -1), (2500, -1), (3000, -1), (3500, 1), (4485, 1), (5000, 1), (10000, 1)])
+def test_shared_memory_is_favoured_while_three_blocks_fit(host, n, sign):
+    """A full panel's class above N=2048 keeps shared memory, though it times
+    like the workspace when alone, where three blocks of four ants (8 n bytes of
+    coordinates; per ant 4 n of tour and inverse, n / 4 of bits) fit on an SM,
+    and the workspace elsewhere; a panel that is not full goes by the times."""
+    host.shared_factor.restype = C.c_float
+    words = (n + 31) // 32
+    block = (8 * n + 15) // 16 * 16 + 4 * ((4 * ((n + 7) // 8 * 8) + 8 * words + 15) // 16 * 16)
+    assert host.shared_factor(0, block) == 1.0
+    assert np.sign(host.shared_factor(1, block) - 1.0) == sign
 
 
 @pytest.mark.gpu
