@@ -315,6 +315,16 @@ def run_reference(args, rank: int) -> None:
     print(json.dumps(line), flush=True)
 
 
+def follow_batches(setting: int, plan: int) -> str:
+    """How the ants take parent-following steps, from the setting and the engine's launch plan (which
+    has 1 for every panel with batches always on, full or not)."""
+    if plan == 0:
+        return "off"
+    if setting == 2:
+        return "always"
+    return {1: "by colony, one-wave build", 2: "by colony, full-panel build"}[plan]
+
+
 def _engine(wl: Workload, device: int, follow: int = 0):
     import gplsaco_gb300 as g
     settings = g.FixedFacoSettings(ants=wl.ants, primary_width=wl.k, backup_width=wl.b, ls_width=wl.w,
@@ -469,7 +479,7 @@ def run_gb300(args, rank: int, world: int) -> None:
                    "iterations_per_step": per_step,
                    "timed_iterations": [0, window],
                    "warmup": "W steps of a separate evaluation; the timed one starts from the initial tours",
-                   "colony_chains": plan["chains"], "follow_batches": {0: "off", 1: "one-wave build", 2: "full-panel build"}[plan["follow"]],
+                   "colony_chains": plan["chains"], "follow_batches": follow_batches(args.follow, plan["follow"]),
                    "registration_seconds": registration_s, "size_classes": classes},
         "e2e": {"value": e2e_value, "unit": "ant-tours+LS/s", "h2d_bytes_per_step": h2d * per_step / e2e_iters,
                 "d2h_bytes_per_step": d2h * per_step / e2e_iters, "iterations": e2e_iters,
