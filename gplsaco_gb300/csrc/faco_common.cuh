@@ -119,16 +119,6 @@ __device__ __forceinline__ double u53(std::uint32_t hi, std::uint32_t lo) {
 
 // Counter layout: (step, ant, batch, tag).  tag 0 construction uniform,
 // 1 start node, 2 colony source draw (ant = 0xffffffff).
-__device__ __forceinline__ double step_uniform(unsigned long long key, std::uint32_t batch, std::uint32_t ant,
-                                               std::uint32_t step) {
-    const uint4v r = philox4x32(step, ant, batch, 0, (std::uint32_t)key, (std::uint32_t)(key >> 32));
-    return u53(r.x, r.y);
-}
-__device__ __forceinline__ std::uint32_t start_node(unsigned long long key, std::uint32_t batch,
-                                                    std::uint32_t ant, std::uint32_t n) {
-    const uint4v r = philox4x32(0, ant, batch, 1, (std::uint32_t)key, (std::uint32_t)(key >> 32));
-    return (std::uint32_t)(((unsigned long long)r.x * n) >> 32);
-}
 __device__ __forceinline__ double source_uniform(unsigned long long key, std::uint32_t batch) {
     const uint4v r = philox4x32(0, 0xffffffffu, batch, 2, (std::uint32_t)key, (std::uint32_t)(key >> 32));
     return u53(r.x, r.y);
@@ -221,7 +211,7 @@ struct ColonyView {
     node_t* archive;               // [2 sides][4 slots][tour, positions][n_pad]
     unsigned long long* ant_ids;   // [ants][2] fingerprints of the batch's tours
     std::uint32_t* ant_p0;         // [ants] position of node 0 in each tour
-    std::uint32_t* walk;           // construction steps per ant of the last iteration (null: not kept)
+    std::uint32_t* walk;           // construction steps per ant of the last iteration
     node_t* parent_pos;            // [n_pad] inverse of `parent` (null: not kept, the ants build their own)
 };
 
