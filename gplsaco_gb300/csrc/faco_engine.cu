@@ -1573,6 +1573,23 @@ int faco_restore(faco_engine* e, const void* buffer, uint64_t bytes, uint32_t tr
                 for (std::uint32_t i = 0, n = v.sizes[c], before = tour[at + n - 1]; i < n; before = tour[at + i++])
                     if (near[at + tour[at + i]] != (tour[at + (i + 1 == n ? 0 : i + 1)] | before << 16))
                         throw Error(FACO_EINVAL, "snapshot parent neighbours differ from the parent tour");
+            // the archive's entries in use, their positions, and the start list
+            for (std::size_t c = 0, at = 0; ref && c < v.sizes.size(); at += faco::pad8(v.sizes[c]), ++c) {
+                const std::uint32_t n = v.sizes[c], n_pad = faco::pad8(n);
+                faco::RefControl ctl;
+                std::memcpy(&ctl, refs + c * sizeof ctl, sizeof ctl);
+                bool sound = ctl.side <= 1 && ctl.archive_size <= faco::kArchive && ctl.start_count <= faco::kRegionNodes;
+                for (std::uint32_t i = 0; sound && i < ctl.start_count; ++i) sound = ctl.start_nodes[i] < n;
+                std::vector<faco::node_t> entry(2 * n_pad), position(n);   // a tour and its positions
+                for (std::uint32_t slot = 0; sound && slot < ctl.archive_size; ++slot) {
+                    const std::size_t row = 16 * at + (ctl.side * faco::kArchive + slot) * entry.size();
+                    std::memcpy(entry.data(), archives + row * sizeof(faco::node_t), entry.size() * sizeof(faco::node_t));
+                    sound = faco::host_inverse(entry.data(), n, position.data()) &&
+                            std::equal(position.begin(), position.end(), entry.begin() + n_pad) &&
+                            ctl.archive_p0[slot] == position[0];
+                }
+                if (!sound) throw Error(FACO_EINVAL, "snapshot archive is not one of tours");
+            }
             put(e->parent_pos.get(), reinterpret_cast<const unsigned char*>(inverse.data()),
                 h.node_total * sizeof(faco::node_t));
             put(e->epoch.get(), epoch, h.node_total * sizeof(faco::node_t));

@@ -277,7 +277,7 @@ int faco_begin_programs(faco_engine* engine, const uint64_t* instance_keys, cons
  * buffer NULL it only reports the size in *bytes.  faco_restore begins a
  * stepwise evaluation from such a snapshot on an engine with the same
  * settings and the same instances registered (coordinates are checked, and that
- * the parent, epoch and global rows are tours);
+ * the parent, epoch, global and archive rows are tours);
  * stepping it continues the saved run bit for bit.  Trace rows are indexed
  * by absolute iteration. */
 int faco_snapshot(faco_engine* engine, void* buffer, uint64_t capacity, uint64_t* bytes);

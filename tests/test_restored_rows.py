@@ -102,3 +102,47 @@ def test_broken_rows_are_refused(engine_lib, workspace):
     assert np.array_equal(got["costs"], want["costs"])
     assert all(np.array_equal(a, b) for a, b in zip(got["tours"], want["tours"]))
     e.close()
+
+
+@pytest.mark.gpu
+def test_broken_archive_is_refused(engine_lib):
+    """The 12-feature controller's archive (the snapshot's last rows: two sides of
+    four tours with their positions) and its start list."""
+    import gplsaco_gb300 as g
+    n, pad = 30, 32
+    keys, seeds = np.array([4], np.uint64), np.array([1], np.uint64)
+    program = dict(ir_version=1, numeric_spec_id=1, feature_spec_id=2, opcode=[0], operand=[0], constant_bits=[])
+    e = g.FacoBatchEngine(n, 1, g.FixedFacoSettings(ants=9, retention=0.9))
+    e.register_problem(4, _cases.uniform_instance(n, seed=3).astype(np.float64))
+    e.begin_programs(keys, seeds, [program], total_iterations=20)
+    e.step(7)
+    state = e.capture_state().to_bytes()
+    e.step(5)
+    want = e.finish()
+    rows = len(state) - 8 - 2 * 16 * pad
+    body = bytearray(state[:-8])
+    # the controller state before the rows ends: size, side, alternative, mask, start count, reserved,
+    # positions of node 0 [4], start nodes [16]
+    tail = struct.Struct("<6I4I16H")
+    control = rows - tail.size
+    size, side, _, _, _, _, *p0 = tail.unpack_from(body, control)
+    at = rows + 2 * 4 * 2 * pad * side
+    assert 1 <= size <= 4 and side <= 1
+    tour = np.frombuffer(bytes(body), np.uint16, n, at)
+    assert np.array_equal(np.sort(tour), np.arange(n)) and tour[p0[0]] == 0
+    breaks = {"node": (at, struct.pack("<H", n)), "twice": (at, struct.pack("<H", int(tour[1]))),
+              "position": (at + 2 * pad + 2 * 5, struct.pack("<H", n)), "size": (control, struct.pack("<I", 5)),
+              "side": (control + 4, struct.pack("<I", 2)), "starts": (control + 16, struct.pack("<I", 17)),
+              "zero": (control + 24, struct.pack("<I", n))}
+    for where, value in breaks.values():
+        broken = bytearray(body)
+        broken[where:where + len(value)] = value
+        broken += struct.pack("<Q", _fnv1a(broken))
+        with pytest.raises(ValueError, match="snapshot archive"):
+            e.restore_state(g.CountedState(bytes(broken)))
+    e.restore_state(g.CountedState(state))
+    e.step(5)
+    got = e.finish()
+    assert np.array_equal(got["costs"], want["costs"])
+    assert all(np.array_equal(a, b) for a, b in zip(got["tours"], want["tours"]))
+    e.close()
